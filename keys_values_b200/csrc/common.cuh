@@ -202,6 +202,17 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// True in one lane of a fully active warp. The branch of an MMA issuer is taken on this and not on the lane index: the
+// compiler then knows that one thread runs it and keeps the descriptors in uniform registers. M = 128, N = 64, K = 16
+// MMAs with A in TMEM, issued back to back by a warp alone on the SM: 32 cycles each against 45 under `lane == 0`
+// (N = 128: 64 both ways, but the moves compete with the compute warps for issue slots: in the attention backward four
+// MMAs held their issuer 75 cycles instead of 318).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
+}
+
 // D[tmem] (+)= A[smem desc] · B[smem desc]; issued by ONE thread.
 __device__ __forceinline__ void umma_f16_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(

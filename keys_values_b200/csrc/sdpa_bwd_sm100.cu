@@ -1,23 +1,26 @@
-// SDPA backward for sm_100a (bf16, head size 128), mask from token positions.
+// SDPA backward for sm_100a (bf16, head size 128 or 64), mask from token positions: every score tile is formed ONCE.
 //
-// Given dO, the forward's O and log-sum-exp, computes
-//   dQ (B,H,T,D) bf16, and accumulates dK, dV into fp32 cache-shaped buffers (B,G,C,D).
-// Two launches of one kernel template, so that every output tile has exactly one
-// owner CTA (no atomics, deterministic):
-//   MODE_DQ : CTA = 128 query rows (positions x heads of a KV group), streams KV slots
-//             S = Q K^T, dP = dO V^T  ->  dS = P (dP − δ) scale  ->  dQ += dS K
-//   MODE_DKV: CTA = 128 KV slots, streams query rows
-//             S^T = K Q^T, dP^T = V dO^T -> P^T, dS^T -> dV += P^T dO, dK += dS^T Q
-// Both are the same pipeline. A fixed "row" tile has two K-major operands (R1, R2) in shared
-// memory. The streamed "column" operands (C1, C2) arrive by TMA in units of 64 columns through a
-// 4-stage ring. For every unit, X = R1 C1^T and Y = R2 C2^T (128 x 64, fp32) are formed in one of
-// two TMEM buffers; the 256 compute threads (TMEM lane = row) turn them into bf16 P and dS, which
-// they write back into the same TMEM columns; the accumulating MMAs then take P / dS as their
-// A operand straight from TMEM and the column operands, from the same shared memory, as
-// MN-major B operands (acc1 += P C2, acc2 += dS C1). P and dS never touch shared memory, whose
-// bandwidth is what bounds this kernel. MMAs of one thread execute in issue order, so the X/Y
-// MMAs of unit u+2, which overwrite the buffer of unit u, are issued after the accumulating
-// MMAs of unit u. δ = rowsum(dO ⊙ O) comes from a small kernel.
+// Given dO, the forward's O and log-sum-exp, computes dQ (B,H,T,D) bf16, and accumulates dK, dV into fp32 cache-shaped
+// buffers (B,G,C,D).
+//   dkv kernel : CTA = 128 KV slots, streams query tiles of 128 packed rows (npos positions x gs heads, head major)
+//                S^T = K Q^T, dP^T = V dO^T  ->  P^T, dS^T  ->  dV += P^T dO, dK += dS^T Q;  dS (bf16) -> workspace
+//   dq kernel  : CTA = 128 query rows, streams KV tiles: dQ += dS K, a product without any softmax in it
+//
+// Why this split. Forming S and dP in a launch for dQ and again in one for dK / dV (7 GEMM-equivalents, in units of 64
+// columns whose M = 128, N = 64 MMAs re-read the 128-row A operand from shared memory for half the arithmetic) took
+// 1.14 ms for 1024 queries x 32 heads over 16384 slots. Here S and dP are formed once, the five necessary products are
+// all that is left, and S and dP have ONE buffer of 128 TMEM columns each beside dV and dK. Two chains, one issuer thread
+// and one accumulator each, keep the tensor pipe busy:
+//     thread A:  wait P(i)  -> dV += P(i) dO(i),  S(i+1)          thread B:  wait dS(i) -> dK += dS(i) Q(i),  dP(i+1)
+// so that the exponentials of a tile run under dK / dP and the products P (dP − δ) under dV / S. S goes in two halves of
+// 64 columns, so that the exponentials of one half overlap dV and the next S of the other. Measured: 0.81 ms back to back
+// under the power cap, 0.69 ms in short runs (dkv 0.48, dq 0.19). dkv: 3220 cycles a tile (2304 of MMA, of which shared
+// memory serves most; compute chain: exponentials 1300 of 1024 at the special-function rate, dS 550, its stores 700);
+// dq: 5.8 TB/s of dS.
+// dS passes through memory (32 KB written and read per tile) instead of being reduced into dQ by atomics: a coalesced
+// red.add.f32 of the 64 KB dQ tile was measured at 5.9 TB/s over the chip, no faster than the two 32 KB passes, and its
+// order is not fixed. Every output has one owner and a fixed order of sums: gradients are the same run to run.
+// The workspace is bounded (BO_DS_LIMIT): larger calls go in rounds over query tiles, then over (sequence, group) pairs.
 //
 // Replaces the blocked fp32 PyTorch backward of the reference
 // (keys_values/attention/sdpa_op.py:31-251) and the library SDPA backward it otherwise uses.
@@ -28,43 +31,42 @@
 #include "common.cuh"
 #include "kvb200.h"
 
+extern "C" int kvb_att_tile_minmax(const int32_t* token_pos, int32_t* tmin, int32_t* tmax, int B, int G, int L, long long tp_sb,
+                                   long long tp_sg, int tile, void* stream);
+
 namespace kvb {
 
-constexpr int BW_TILE_BYTES = 128 * 128 * 2;   // row operand: two 64-feature chunks of [128 rows x 128 B]
-constexpr int BW_UNIT_BYTES = 64 * 128 * 2;    // column operand of one unit: two chunks of [64 rows x 128 B]
-constexpr int BW_STAGES = 4;                   // ring of column units (C1 | C2 per stage)
-constexpr int BW_THREADS = 352;                // TMA warp + MMA warp (even units) + 8 compute warps + MMA warp (odd units)
-enum { MODE_DQ = 0, MODE_DKV = 1 };
+constexpr int BO_TILE = 128 * 128 * 2;       // 32 KB: two 64-feature chunks of [128 rows x 128 B]
+constexpr int BO_CHUNK = BO_TILE / 2;
+constexpr int BO_QSTAGES = 3, BO_OSTAGES = 2;  // Q lives from S(i) to dK(i), dO from dP(i) to dV(i)
+constexpr int BO_THREADS = 384;              // producer, issuer A, issuer B, idle, 8 compute warps
+constexpr int BO_QK_STAGES = 3;              // dq kernel: dS tile | K tile per stage
+constexpr int BO_DQ_THREADS = 192;           // producer, issuer, 4 epilogue warps
 
-struct BwSmem {
-  static constexpr int R1 = 0;
-  static constexpr int R2 = R1 + BW_TILE_BYTES;
-  static constexpr int C = R2 + BW_TILE_BYTES;                    // per stage: C1 | C2
-  static constexpr int STATS = C + BW_STAGES * 2 * BW_UNIT_BYTES; // tp[128] | nlse[2][128] | ndls[2][128]
-  static constexpr int FLAGS = STATS + 512 + 1024 + 1024;         // one byte per column tile: bit 0 active, bit 1 masked
-  static constexpr int NFLAGS = 4096;
-  static constexpr int BAR = FLAGS + NFLAGS;
-  static constexpr int TOTAL = BAR + 256 + 1024;
+struct BoSmem {
+  static constexpr int K = 0;
+  static constexpr int V = K + BO_TILE;
+  static constexpr int Q = V + BO_TILE;
+  static constexpr int O = Q + BO_QSTAGES * BO_TILE;
+  static constexpr int STAT = O + BO_OSTAGES * BO_TILE;  // two slots of −lse·log2(e)[128] | −delta·scale[128]
+  static constexpr int BAR = STAT + 2 * 1024;
+  static constexpr int TOTAL = BAR + 256;
+  static constexpr int ROW = 256 + 16;  // epilogue: padded half rows of 64 fp32, one buffer of 32 rows per compute warp
 };
+static_assert(BoSmem::TOTAL <= 232448, "shared memory of the dkv kernel exceeds the limit of a CTA");
+static_assert(8 * 32 * BoSmem::ROW <= BO_QSTAGES * BO_TILE, "epilogue buffers alias the Q ring");
 
-struct BwParams {
+struct BoParams {
   const int32_t* token_pos;
-  const int32_t* tile_min;
+  const int32_t* tile_min;   // (B,G,nT)
   const int32_t* tile_max;
-  const float* lse;     // (B,H,T) natural log
-  const float* delta;   // (B,H,T)
-  __nv_bfloat16* dq;    // (B,H,T,D)
-  float* dk;            // (B,G,C,D) accumulated
+  const float* stats;        // (B·G, nQT, 2, 128): −lse·log2(e) (−inf: no query), −delta·scale
+  __nv_bfloat16* ds;         // workspace of the round: (pairs, nT, nq) tiles of [16 units of 8 rows][128 slots][8]
+  __nv_bfloat16* dq;         // (B,H,T,D)
+  float* dk;                 // (B,G,C,D) accumulated
   float* dv;
-  int B, H, G, T, L, nT, nQT, gs, npos;
-  // Query rows are packed head-major: a 128-row tile of the dQ launch holds npos = 128 / gs (rounded down) positions
-  // x gs heads (rows_used of 128 rows), a 64-column unit of the dK/dV launch holds hnpos positions x u_heads
-  // heads (cols_used of 64 columns); a column tile of the dK/dV launch is two units and spans npos_col positions.
-  int rows_used, hnpos, cols_used, npos_col, nCT;
-  // Unit h of a column tile holds u_heads heads x hnpos positions, from head h·u_dh and position h·u_dp of the tile:
-  // half of the heads over all positions of the tile when the group size is an even power of two (u_dh = gs / 2,
-  // u_dp = 0), all heads over half of the positions otherwise (u_dh = 0, u_dp = hnpos).
-  int u_heads, u_dh, u_dp;
+  int G, H, T, L, nT, nQT, gs, npos, rows_used;
+  int bg0, q0, nq;           // this round: first (sequence, group) pair, query tiles [q0, q0 + nq)
   long long tp_sb, tp_sg, dk_sb, dk_sg;
   float scale, scale_log2;
   int input_pos;
@@ -78,45 +80,58 @@ struct BwParams {
   int trace_cap;
 };
 
-// Timeline event of one role (1 MMA issuer, 2 first compute warp) of CTA 0.
-#define BW_TRACE(role, tag)                                               \
+// Timeline event of one role (1 MMA issuer, 2 first compute warp) of CTA 0; tr_n starts at BO_TRACE_OFF everywhere else.
+#define BO_TRACE_OFF (1 << 30)
+#define BO_TRACE(role, tag)                                               \
   do {                                                                    \
-    if (p.trace && blockIdx.x == 0 && tr_n < p.trace_cap) {               \
+    if (tr_n < p.trace_cap) {                                             \
       p.trace[((role) * p.trace_cap + tr_n) * 2] = (long long)(tag);      \
       p.trace[((role) * p.trace_cap + tr_n) * 2 + 1] = clock64();         \
       ++tr_n;                                                             \
     }                                                                     \
   } while (0)
 
-__device__ __forceinline__ float bw_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-// hardware tanh, as in the forward kernels (P must be recomputed from the same capped scores)
-__device__ __forceinline__ float bw_tanh(float z) {
-  float t;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(z));
-  return t;
+__device__ __forceinline__ int bo_qpos_max(const BoParams& p, int qt) { return p.input_pos + min((qt + 1) * p.npos, p.T) - 1; }
+// some query of tile qt sees some slot of a KV tile whose token positions span [tmin, tmax]
+template <bool GEN>
+__device__ __forceinline__ bool bo_active(const BoParams& p, int qt, int tmin, int tmax) {
+  return tmin <= bo_qpos_max(p, qt) && (!GEN || p.window <= 0 || tmax > p.input_pos + qt * p.npos - p.window);
 }
 
-// delta[b,h,t] = sum_d dO[b,t,h,d] * O[b,t,h,d]
-// With dOt the kernel also leaves a head-major copy dOt[b,h,t,:] of dO (which it reads anyway): the TMA boxes of the
-// two launches then read runs of consecutive positions of one head, as they do for Q.
+// Statistics per packed query row and a head-major copy of dO, one warp per packed row:
+// stats[bg][qt][0][row] = −lse·log2(e), stats[bg][qt][1][row] = −scale·sum_d dO·O; rows without a query: −inf, 0 (P = dS = 0).
 template <int HD>
-__global__ void att_delta_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O,
-                                 float* __restrict__ delta, __nv_bfloat16* __restrict__ dOt, int B, int T, int H) {
-  const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (row >= (long long)B * T * H) return;
+__global__ void bo_stats_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O, const float* __restrict__ lse,
+                                float* __restrict__ stats, __nv_bfloat16* __restrict__ dOt, int B, int G, int H, int T, int gs,
+                                int npos, int nQT, float scale) {
+  const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int row = (int)(w & 127);
+  const long long tile = w >> 7;  // (bg, qt)
+  if (tile >= (long long)B * G * nQT) return;
   const int lane = threadIdx.x & 31;
+  const int qt = (int)(tile % nQT);
+  const int bg = (int)(tile / nQT);
+  const int b = bg / G, g = bg % G;
+  const int hq = row / npos, t = qt * npos + row % npos;
+  float* st = stats + tile * 256 + row;
+  if (hq >= gs || t >= T) {
+    if (lane == 0) {
+      st[0] = -INFINITY;
+      st[128] = 0.f;
+    }
+    return;
+  }
+  const int h = g * gs + hq;
   constexpr int PER = HD / 32;  // features per lane: 4 (one 8-byte access) or 2 (one 4-byte access)
+  const long long src = (((long long)b * T + t) * H + h) * HD + lane * PER;
+  const long long hrow = ((long long)b * H + h) * T + t;
   uint2 a = make_uint2(0, 0), o = make_uint2(0, 0);
   if (PER == 4) {
-    a = *reinterpret_cast<const uint2*>(dO + row * HD + lane * 4);
-    o = *reinterpret_cast<const uint2*>(O + row * HD + lane * 4);
+    a = *reinterpret_cast<const uint2*>(dO + src);
+    o = *reinterpret_cast<const uint2*>(O + src);
   } else {
-    a.x = *reinterpret_cast<const uint32_t*>(dO + row * HD + lane * 2);
-    o.x = *reinterpret_cast<const uint32_t*>(O + row * HD + lane * 2);
+    a.x = *reinterpret_cast<const uint32_t*>(dO + src);
+    o.x = *reinterpret_cast<const uint32_t*>(O + src);
   }
   const __nv_bfloat162* ap = reinterpret_cast<const __nv_bfloat162*>(&a);
   const __nv_bfloat162* op = reinterpret_cast<const __nv_bfloat162*>(&o);
@@ -127,116 +142,106 @@ __global__ void att_delta_kernel(const __nv_bfloat16* __restrict__ dO, const __n
     s += x.x * y.x + x.y * y.y;
   }
   s = warp_sum(s);
-  const int h = (int)(row % H);
-  const long long bt = row / H;
-  const int t = (int)(bt % T);
-  const int b = (int)(bt / T);
-  const long long hrow = ((long long)b * H + h) * T + t;
-  if (dOt) {
-    if (PER == 4) *reinterpret_cast<uint2*>(dOt + hrow * HD + lane * 4) = a;
-    else *reinterpret_cast<uint32_t*>(dOt + hrow * HD + lane * 2) = a.x;
+  if (PER == 4) *reinterpret_cast<uint2*>(dOt + hrow * HD + lane * 4) = a;
+  else *reinterpret_cast<uint32_t*>(dOt + hrow * HD + lane * 2) = a.x;
+  if (lane == 0) {
+    st[0] = -lse[hrow] * 1.4426950408889634f;
+    st[128] = -s * scale;
   }
-  if (lane == 0) delta[hrow] = s;
 }
 
-// tmR1/tmR2: row operands (boxes of 128 rows); tmC1/tmC2: column operands (boxes of 64 rows).
-//   MODE_DQ : R1 = Q, R2 = dO, C1 = K, C2 = V      MODE_DKV: R1 = K, R2 = V, C1 = Q, C2 = dO
-// GEN: sliding window and / or soft-capping are in use (separate instantiations, so that the plain kernels keep their
-// register allocation)
-// HD: head size, 128 or 64 (row operands and units of one 64-feature chunk, half as many K steps for X / Y,
-// accumulators of 64 columns)
-template <int MODE, bool GEN, int HD>
-__global__ void __launch_bounds__(BW_THREADS, 1)
-sdpa_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ CUtensorMap tmR2,
-                const __grid_constant__ CUtensorMap tmC1, const __grid_constant__ CUtensorMap tmC2, const BwParams p) {
-  using S = BwSmem;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+__device__ __forceinline__ float bo_exp2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// hardware tanh, as in the forward kernels (P must be recomputed from the same capped scores)
+__device__ __forceinline__ float bo_tanh(float z) {
+  float t;
+  asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(z));
+  return t;
+}
+
+// Bits of the columns [c0, c0 + 32) whose position lies before `th` positions into the tile (columns are head major,
+// npos per head): the queries that may not see a token `th` positions beyond the first one of the tile.
+__device__ __forceinline__ uint32_t bo_hidden(int c0, int npos, int th) {
+  uint32_t bits = 0;
+  for (int lo = (c0 / npos) * npos - c0; lo < 32; lo += npos) {
+    const int a = max(lo, 0), e = min(lo + th, 32);
+    if (e > a) bits |= (0xffffffffu >> (32 - (e - a))) << a;
+  }
+  return bits;
+}
+
+// GEN: sliding window and / or soft-capping are in use (instantiations of their own, so that the plain kernels keep their
+// registers). HD: head size, 128 or 64 (tiles of one 64-feature chunk, half as many K steps, accumulators of 64 columns).
+template <bool GEN, int HD>
+__global__ void __launch_bounds__(BO_THREADS, 1)
+bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+               const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmO, const BoParams p) {
+  using S = BoSmem;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  if (smem_u32(smem) & 1023u) {  // swizzled tiles need a 1024-byte aligned window: report, do not run
+    if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, STATUS_TIMEOUT_MISC);
+    return;
+  }
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::BAR);
-  uint64_t* r_full = bars + 0;
-  uint64_t* c_full = bars + 1;     // [4]
-  uint64_t* c_empty = bars + 5;    // [4]
-  uint64_t* xy_full = bars + 9;    // [2]
-  uint64_t* pds_full = bars + 11;  // [2]
-  uint64_t* acc_full = bars + 13;
-  uint64_t* grp_bar = bars + 14;
-  uint64_t* rows_ready = bars + 15;  // accumulators zeroed (and, MODE_DQ, the row operands moved to TMEM)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  uint64_t* k_full = bars + 0;
+  uint64_t* v_full = bars + 1;
+  uint64_t* q_full = bars + 2;     // [3]
+  uint64_t* q_empty = bars + 5;    // [3]
+  uint64_t* o_full = bars + 8;     // [2]
+  uint64_t* o_empty = bars + 10;   // [2] dV (thread A) and dP (thread B) have read dO
+  uint64_t* st_full = bars + 12;   // [2]
+  uint64_t* x_full = bars + 14;    // [2] halves of 64 columns
+  uint64_t* p_full = bars + 16;    // [2]
+  uint64_t* y_full = bars + 18;
+  uint64_t* ds_full = bars + 19;
+  uint64_t* acc_full = bars + 20;  // one commit per issuer
+  uint64_t* a_issued = bars + 21;  // thread A has issued S(i + 1)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* stat_nlse = reinterpret_cast<float*>(smem + S::STATS + 512);  // MODE_DKV: [2][128] −lse·log2(e) of the query tile
-  float* stat_ndls = reinterpret_cast<float*>(smem + S::STATS + 1536); // MODE_DKV: [2][128] −delta·scale of the query tile
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n_row_tiles = MODE == MODE_DQ ? p.nQT : p.nT;
-  const int qtile_pos = MODE == MODE_DQ ? p.npos : p.npos_col;  // positions per query tile of this launch
-  const int rt = blockIdx.x % n_row_tiles;                 // row tile: query tile (DQ) or KV tile (DKV)
-  const int g = (blockIdx.x / n_row_tiles) % p.G;
-  const int b = blockIdx.x / (n_row_tiles * p.G);
-  const int32_t* tmin = p.tile_min + ((long long)b * p.G + g) * p.nT;
-  const int32_t* tmax = p.tile_max + ((long long)b * p.G + g) * p.nT;
-  const int n_col_tiles = MODE == MODE_DQ ? p.nT : p.nCT;
+  const int kt = blockIdx.x % p.nT;
+  const int lbg = blockIdx.x / p.nT;
+  const int bg = p.bg0 + lbg;
+  const int b = bg / p.G, g = bg % p.G;
+  // Query tiles that see this KV tile: without a window all from one on (its oldest token), with one up to another (its newest).
+  const int tmin = p.tile_min[(long long)bg * p.nT + kt], tmax = p.tile_max[(long long)bg * p.nT + kt];
+  int q_first = p.q0, q_end = p.q0 + p.nq;
+  while (q_first < q_end && !bo_active<GEN>(p, q_first, tmin, tmax)) ++q_first;
+  if (GEN)
+    while (q_end > q_first && !bo_active<GEN>(p, q_end - 1, tmin, tmax)) --q_end;
+  const int n = q_end - q_first;
+  if (n <= 0) return;
 
-  // (kv tile t, query tile qt) is active iff some slot of t is visible to some query of qt
-  auto qpos_min_of = [&](int qt) { return p.input_pos + qt * qtile_pos; };
-  auto qpos_max_of = [&](int qt) { return p.input_pos + min((qt + 1) * qtile_pos, p.T) - 1; };
-  // with a window, a tile is also inactive when its newest token has left the window of the first query, and
-  // masked when its oldest token has left the window of the last query
-  const int win = GEN ? p.window : 0;
-  auto active_g = [&](int ct) -> bool {
-    const int kt = MODE == MODE_DQ ? ct : rt, qt = MODE == MODE_DQ ? rt : ct;
-    return tmin[kt] <= qpos_max_of(qt) && (win <= 0 || tmax[kt] > qpos_min_of(qt) - win);
-  };
-  auto masked_g = [&](int ct) -> bool {
-    const int kt = MODE == MODE_DQ ? ct : rt, qt = MODE == MODE_DQ ? rt : ct;
-    return tmax[kt] > qpos_min_of(qt) || (win > 0 && tmin[kt] <= qpos_max_of(qt) - win);
-  };
-  // the flags of the column tiles are kept in shared memory so that no role reads global memory
-  // inside its tile loop
-  uint8_t* tflags = smem + S::FLAGS;
-  for (int ct = threadIdx.x; ct < n_col_tiles && ct < S::NFLAGS; ct += BW_THREADS)
-    tflags[ct] = (uint8_t)((active_g(ct) ? 1 : 0) | (masked_g(ct) ? 2 : 0));
-  auto active = [&](int ct) -> bool { return ct < S::NFLAGS ? (tflags[ct] & 1) != 0 : active_g(ct); };
-  auto masked = [&](int ct) -> bool { return ct < S::NFLAGS ? (tflags[ct] & 2) != 0 : masked_g(ct); };
-  auto next_active = [&](int ct) -> int {
-    while (ct < n_col_tiles && !active(ct)) ++ct;
-    return ct;
-  };
-
-  // Rows that no TMA box ever writes (group sizes that do not divide the tile: 128 − rows_used rows of the row
-  // operands in the dQ launch, 64 − cols_used rows of every streamed unit in the dK/dV launch) are zeroed once: they
-  // enter MMAs as operand rows, and 0 · anything finite is 0 while stale shared memory could hold NaN patterns.
-  if (MODE == MODE_DQ && p.rows_used < 128) {
-    const int n16 = (128 - p.rows_used) * 8;  // 16-byte pieces per 64-feature chunk
-    constexpr int NCH = HD / 64;
-    for (int i = threadIdx.x; i < 2 * NCH * n16; i += BW_THREADS) {
-      uint8_t* chunk = smem + ((i / n16) / NCH == 0 ? S::R1 : S::R2) + ((i / n16) % NCH) * (BW_TILE_BYTES / 2);
-      *reinterpret_cast<uint4*>(chunk + p.rows_used * 128 + (i % n16) * 16) = make_uint4(0, 0, 0, 0);
-    }
-    fence_proxy_async_smem();
-  }
-  if (MODE == MODE_DKV && p.cols_used < 64) {
-    const int n16 = (64 - p.cols_used) * 8;
-    constexpr int NCH = HD / 64;
-    for (int i = threadIdx.x; i < BW_STAGES * 2 * NCH * n16; i += BW_THREADS) {
-      const int idx = i / n16;  // (stage, operand C1 | C2, 64-feature chunk)
-      uint8_t* chunk = smem + S::C + (idx / NCH) * BW_UNIT_BYTES + (idx % NCH) * (BW_UNIT_BYTES / 2);
-      *reinterpret_cast<uint4*>(chunk + p.cols_used * 128 + (i % n16) * 16) = make_uint4(0, 0, 0, 0);
-    }
+  if (p.rows_used < 128) {  // rows that no TMA box writes enter MMAs as operand rows: finite zeros
+    const int n16 = (128 - p.rows_used) * 8;
+    for (int i = threadIdx.x; i < (BO_QSTAGES + BO_OSTAGES) * 2 * n16; i += BO_THREADS)
+      *reinterpret_cast<uint4*>(smem + S::Q + (i / n16) * BO_CHUNK + p.rows_used * 128 + (i % n16) * 16) = make_uint4(0, 0, 0, 0);
     fence_proxy_async_smem();
   }
   if (threadIdx.x == 0) {
-    mbar_init(r_full, 1);
-    for (int s = 0; s < BW_STAGES; ++s) {
-      mbar_init(&c_full[s], 1);
-      mbar_init(&c_empty[s], 1);
+    mbar_init(k_full, 1);
+    mbar_init(v_full, 1);
+    for (int s = 0; s < BO_QSTAGES; ++s) {
+      mbar_init(&q_full[s], 1);
+      mbar_init(&q_empty[s], 1);
     }
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&xy_full[s], 1);
-      mbar_init(&pds_full[s], 8);
+    for (int s = 0; s < BO_OSTAGES; ++s) {
+      mbar_init(&o_full[s], 1);
+      mbar_init(&o_empty[s], 2);
+      mbar_init(&st_full[s], 1);
     }
-    mbar_init(acc_full, 2);  // one commit per MMA issuer
-    mbar_init(grp_bar, 256);
-    mbar_init(rows_ready, 8);
+    for (int h = 0; h < 2; ++h) {
+      mbar_init(&x_full[h], 1);
+      mbar_init(&p_full[h], 8);
+    }
+    mbar_init(y_full, 1);
+    mbar_init(ds_full, 8);
+    mbar_init(acc_full, 2);
+    mbar_init(a_issued, 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -248,56 +253,39 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // X buffers: columns [0,64) and [64,128); Y buffers: [128,192) and [192,256); accumulators after
-  // MODE_DQ has one accumulator only; the free 128 columns hold its row operands Q and dO as bf16
-  // pairs (64 columns each), so that the X / Y MMAs take A from TMEM and read only the streamed
-  // columns from shared memory.
-  const uint32_t tmem_X = tmem_base, tmem_Y = tmem_base + 128, tmem_A1 = tmem_base + 256;
-  const uint32_t tmem_A2 = tmem_base + (MODE == MODE_DQ ? 256 : 384);
-  const uint32_t tmem_R1 = tmem_base + 384, tmem_R2 = tmem_base + 448;  // MODE_DQ only
-
-  int n_active = 0;
-  for (int ct = 0; ct < n_col_tiles; ++ct) n_active += active(ct) ? 1 : 0;
+  const uint32_t tmem_X = tmem_base, tmem_Y = tmem_base + 128, tmem_dV = tmem_base + 256, tmem_dK = tmem_base + 384;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0 && n_active > 0) {
-      tma_prefetch_desc(&tmR1);
-      tma_prefetch_desc(&tmR2);
-      tma_prefetch_desc(&tmC1);
-      tma_prefetch_desc(&tmC2);
-      mbar_expect_tx(r_full, MODE == MODE_DQ ? (uint32_t)(4 * p.rows_used * HD) : (uint32_t)(2 * 128 * HD * 2));
-      {
-        const int c1 = MODE == MODE_DQ ? rt * p.npos : rt * 128;
-        const int c2 = MODE == MODE_DQ ? g * p.gs : g;
-        tma_load_4d(smem + S::R1, &tmR1, r_full, 0, c1, c2, b);
-        if (HD == 128) tma_load_4d(smem + S::R1 + BW_TILE_BYTES / 2, &tmR1, r_full, 64, c1, c2, b);
-        tma_load_4d(smem + S::R2, &tmR2, r_full, 0, c1, c2, b);
-        if (HD == 128) tma_load_4d(smem + S::R2 + BW_TILE_BYTES / 2, &tmR2, r_full, 64, c1, c2, b);
-      }
-      uint32_t u = 0;
+    if (lane == 0) {
+      tma_prefetch_desc(&tmQ);
+      tma_prefetch_desc(&tmO);
+      mbar_expect_tx(k_full, 256 * HD);
+      tma_load_4d(smem + S::K, &tmK, k_full, 0, kt * 128, g, b);
+      if (HD == 128) tma_load_4d(smem + S::K + BO_CHUNK, &tmK, k_full, 64, kt * 128, g, b);
       bool ok = true;
-      for (int ct = 0; ct < n_col_tiles && ok; ++ct) {
-        if (!active(ct)) continue;
-        for (int h = 0; h < 2; ++h, ++u) {
-          const int st = u % BW_STAGES;
-          if (!mbar_wait_bounded(&c_empty[st], ((u / BW_STAGES) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_EMPTY)) { ok = false; break; }
-          uint8_t* c1 = smem + S::C + st * 2 * BW_UNIT_BYTES;
-          uint8_t* c2 = c1 + BW_UNIT_BYTES;
-          int x1, x2;  // coordinates 1 and 2 of the 64-row box
-          if (MODE == MODE_DQ) {
-            x1 = ct * 128 + h * 64;
-            x2 = g;
-          } else {  // unit h of query tile ct
-            x1 = ct * p.npos_col + h * p.u_dp;
-            x2 = g * p.gs + h * p.u_dh;
-          }
-          mbar_expect_tx(&c_full[st], MODE == MODE_DQ ? (uint32_t)(2 * 64 * HD * 2) : (uint32_t)(4 * p.cols_used * HD));
-          tma_load_4d(c1, &tmC1, &c_full[st], 0, x1, x2, b);
-          if (HD == 128) tma_load_4d(c1 + BW_UNIT_BYTES / 2, &tmC1, &c_full[st], 64, x1, x2, b);
-          tma_load_4d(c2, &tmC2, &c_full[st], 0, x1, x2, b);
-          if (HD == 128) tma_load_4d(c2 + BW_UNIT_BYTES / 2, &tmC2, &c_full[st], 64, x1, x2, b);
+      for (int i = 0; i < n && ok; ++i) {
+        const int qs = i % BO_QSTAGES, os = i % BO_OSTAGES, t0 = (q_first + i) * p.npos;
+        const uint32_t bytes = (uint32_t)(p.rows_used * HD * 2);
+        if (!(ok = mbar_wait_bounded(&q_empty[qs], ((i / BO_QSTAGES) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_EMPTY))) break;
+        uint8_t* qd = smem + S::Q + qs * BO_TILE;
+        mbar_expect_tx(&q_full[qs], bytes);
+        tma_load_4d(qd, &tmQ, &q_full[qs], 0, t0, g * p.gs, b);
+        if (HD == 128) tma_load_4d(qd + BO_CHUNK, &tmQ, &q_full[qs], 64, t0, g * p.gs, b);
+        if (i == 0) {
+          mbar_expect_tx(v_full, 256 * HD);
+          tma_load_4d(smem + S::V, &tmV, v_full, 0, kt * 128, g, b);
+          if (HD == 128) tma_load_4d(smem + S::V + BO_CHUNK, &tmV, v_full, 64, kt * 128, g, b);
         }
+        if (!(ok = mbar_wait_bounded(&o_empty[os], ((i / BO_OSTAGES) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_EMPTY))) break;
+        uint8_t* od = smem + S::O + os * BO_TILE;
+        mbar_expect_tx(&o_full[os], bytes);
+        tma_load_4d(od, &tmO, &o_full[os], 0, t0, g * p.gs, b);
+        if (HD == 128) tma_load_4d(od + BO_CHUNK, &tmO, &o_full[os], 64, t0, g * p.gs, b);
+        // the slot of these statistics is free once dK(i − 2) has run, which the next Q tile waits for anyway
+        if (i >= 2 && !(ok = mbar_wait_bounded(&q_empty[(i - 2) % BO_QSTAGES], ((i - 2) / BO_QSTAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_EMPTY))) break;
+        mbar_expect_tx(&st_full[i & 1], 1024);
+        bulk_load(smem + S::STAT + (i & 1) * 1024, p.stats + ((long long)bg * p.nQT + q_first + i) * 256, 1024, &st_full[i & 1]);
       }
       if (!ok) {  // let copies in flight land before the CTA's shared memory is released
         long long c0 = clock64();
@@ -305,392 +293,242 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant_
         }
       }
     }
-  } else if (warp == 1 || warp == 10) {
+  } else if (warp == 1 || warp == 2) {
     // ------------------------------------------------------------ MMA issuers
-    // Two threads issue: warp 1 the even units, warp 10 the odd ones. A unit's MMAs (its X / Y pair
-    // and, two units later in the same thread, the accumulating MMAs that read P / dS from the same
-    // TMEM buffer) stay in one thread, so their order is the issue order; the accumulators are
-    // shared by both threads, which is why they are zeroed up front and every MMA accumulates.
-    // While one thread sits in its barrier waits (≈ 250 cycles each, even when satisfied) the other
-    // one keeps the tensor pipe fed.
-    if (lane == 0 && n_active > 0) {
-      const uint32_t par = warp == 1 ? 0u : 1u;
-      constexpr uint32_t idesc_xy = make_idesc_bf16(128, 64, 0, 0);     // both operands K-major
-      constexpr uint32_t idesc_acc = make_idesc_bf16(128, HD, 0, 1);    // A from TMEM, B MN-major
-      const uint32_t r1 = smem_u32(smem + S::R1), r2 = smem_u32(smem + S::R2);
-      const uint32_t cbase = smem_u32(smem + S::C);
-      const uint32_t n_units = 2u * (uint32_t)n_active;
-      bool ok = mbar_wait_bounded(r_full, 0, abort_flag, p.status, STATUS_TIMEOUT_FULL);
-      if (ok) {
-        ok = mbar_wait_bounded(rows_ready, 0, abort_flag, p.status, STATUS_TIMEOUT_FULL);
-        tc_fence_after();
-      }
-      int tr_n = par == 0 ? 0 : (1 << 30);  // only the first issuer records
-      auto wait_c = [&](uint32_t u) -> bool {
-        return mbar_wait_bounded(&c_full[u % BW_STAGES], (u / BW_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL);
-      };
-      auto issue_xy = [&](uint32_t u) -> bool {  // after wait_c(u)
-        const uint32_t st = u % BW_STAGES, hb = u & 1;
-        tc_fence_after();
-        const uint32_t c1 = cbase + st * 2 * BW_UNIT_BYTES, c2 = c1 + BW_UNIT_BYTES;
+    if (elect_one()) {
+      constexpr uint32_t idesc_acc = make_idesc_bf16(128, HD, 0, 1);  // A from TMEM, B MN-major
+      constexpr uint32_t idesc_x = make_idesc_bf16(128, 64, 0, 0), idesc_y = make_idesc_bf16(128, 128, 0, 0);
+      // scores from two K-major tiles in shared memory
+      auto scores = [&](uint32_t d, uint32_t a, uint32_t bm, uint32_t idesc) {
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t a_off = (uint32_t)((kk >> 2) * (BW_TILE_BYTES / 2) + (kk & 3) * 32);
-          const uint32_t b_off = (uint32_t)((kk >> 2) * (BW_UNIT_BYTES / 2) + (kk & 3) * 32);
-          if (MODE == MODE_DQ)
-            umma_f16_ts(tmem_X + 64 * hb, tmem_R1 + 8 * kk, make_smem_desc_sw128(c1 + b_off, 16, 1024), idesc_xy, kk != 0);
-          else
-            umma_f16_ss(tmem_X + 64 * hb, make_smem_desc_sw128(r1 + a_off, 16, 1024), make_smem_desc_sw128(c1 + b_off, 16, 1024),
-                        idesc_xy, kk != 0);
+          const uint32_t off = (uint32_t)((kk >> 2) * BO_CHUNK + (kk & 3) * 32);
+          umma_f16_ss(d, make_smem_desc_sw128(a + off, 16, 1024), make_smem_desc_sw128(bm + off, 16, 1024), idesc, kk != 0);
         }
-#pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t a_off = (uint32_t)((kk >> 2) * (BW_TILE_BYTES / 2) + (kk & 3) * 32);
-          const uint32_t b_off = (uint32_t)((kk >> 2) * (BW_UNIT_BYTES / 2) + (kk & 3) * 32);
-          if (MODE == MODE_DQ)
-            umma_f16_ts(tmem_Y + 64 * hb, tmem_R2 + 8 * kk, make_smem_desc_sw128(c2 + b_off, 16, 1024), idesc_xy, kk != 0);
-          else
-            umma_f16_ss(tmem_Y + 64 * hb, make_smem_desc_sw128(r2 + a_off, 16, 1024), make_smem_desc_sw128(c2 + b_off, 16, 1024),
-                        idesc_xy, kk != 0);
-        }
-        umma_commit(&xy_full[hb]);
-        return true;
       };
-      auto issue_acc = [&](uint32_t u) -> bool {
-        const uint32_t st = u % BW_STAGES, hb = u & 1;
-        if (!mbar_wait_bounded(&pds_full[hb], (u >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL)) return false;
-        BW_TRACE(1, 1200000 + u);
-        tc_fence_after();
-        const uint32_t c1 = cbase + st * 2 * BW_UNIT_BYTES, c2 = c1 + BW_UNIT_BYTES;
-        // A: 16 columns of the unit per step = 8 TMEM columns; the two compute warps of a lane
-        // quarter keep their 32 columns in separate 32-column halves of the buffer.
-        // B: MN-major, 16 rows of the unit per step (2048 B); the 64-feature chunks are LBO apart.
-        // All steps of one accumulator are issued back to back: changing the accumulator between
-        // MMAs costs far more than the MMA itself.
-        if (MODE == MODE_DKV) {
+      auto scores_half = [&](int h, uint32_t bm) {  // columns [64·h, +64) of S
+        scores(tmem_X + (uint32_t)(64 * h), smem_u32(smem + S::K), bm + (uint32_t)(h * 64 * 128), idesc_x);
+        umma_commit(&x_full[h]);
+      };
+      // D += A · B over the 64 query rows of half h, A (P or dS, packed bf16) in TMEM: the two compute warps of a lane
+      // quarter keep their 32 columns as 16 packed ones at columns 0 and 32 of the half
+      auto accumulate = [&](uint32_t d, uint32_t a, uint32_t bm, int h, bool first) {
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            const uint32_t a_col = (uint32_t)(32 * (kk >> 1) + 8 * (kk & 1));
-            const uint32_t b_off = (uint32_t)(kk * 16 * 128);
-            umma_f16_ts(tmem_A1, tmem_X + 64 * hb + a_col, make_smem_desc_sw128(c2 + b_off, BW_UNIT_BYTES / 2, 1024), idesc_acc, 1);
+        for (int u = 0; u < 4; ++u)
+          umma_f16_ts(d, a + (uint32_t)(64 * h + 32 * (u >> 1) + 8 * (u & 1)),
+                      make_smem_desc_sw128(bm + (uint32_t)((4 * h + u) * 16 * 128), BO_CHUNK, 1024), idesc_acc, (first && u == 0) ? 0u : 1u);
+      };
+      auto q_addr = [&](int i) { return smem_u32(smem + S::Q + (i % BO_QSTAGES) * BO_TILE); };
+      auto o_addr = [&](int i) { return smem_u32(smem + S::O + (i % BO_OSTAGES) * BO_TILE); };
+      auto wait_q = [&](int i) { return mbar_wait_bounded(&q_full[i % BO_QSTAGES], (i / BO_QSTAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL); };
+      auto wait_o = [&](int i) { return mbar_wait_bounded(&o_full[i % BO_OSTAGES], (i / BO_OSTAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL); };
+      bool ok;
+      int tr_n = p.trace && blockIdx.x == 0 && warp == 1 ? 0 : BO_TRACE_OFF;
+      if (warp == 1) {
+        ok = mbar_wait_bounded(k_full, 0, abort_flag, p.status, STATUS_TIMEOUT_FULL) && wait_q(0);
+        if (ok) {
+          tc_fence_after();
+          scores_half(0, q_addr(0));
+          scores_half(1, q_addr(0));
+        }
+        for (int i = 0; i < n && ok; ++i) {
+          const bool more = i + 1 < n;
+          if (!(ok = wait_o(i) && (!more || wait_q(i + 1)))) break;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            BO_TRACE(1, 1000000 + 2 * i + h);
+            if (!(ok = mbar_wait_bounded(&p_full[h], i & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL))) break;
+            BO_TRACE(1, 1100000 + 2 * i + h);
+            tc_fence_after();
+            accumulate(tmem_dV, tmem_X, o_addr(i), h, i == 0 && h == 0);
+            if (h == 1) umma_commit(&o_empty[i % BO_OSTAGES]);
+            if (more) scores_half(h, q_addr(i + 1));
+            BO_TRACE(1, 1200000 + 2 * i + h);
+          }
+          if (!ok) break;
+          mbar_arrive(a_issued);
+        }
+      } else {
+        ok = mbar_wait_bounded(v_full, 0, abort_flag, p.status, STATUS_TIMEOUT_FULL) && wait_o(0);
+        if (ok) {
+          tc_fence_after();
+          scores(tmem_Y, smem_u32(smem + S::V), o_addr(0), idesc_y);
+          umma_commit(y_full);
+          umma_commit(&o_empty[0]);
+        }
+        for (int i = 0; i < n && ok; ++i) {
+          const bool more = i + 1 < n;
+          if (!(ok = wait_q(i) && (!more || wait_o(i + 1)))) break;
+          // The next scores go first: the exponentials hang on them, and the tensor pipe serves both threads in turn.
+          if (!(ok = mbar_wait_bounded(a_issued, i & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL))) break;
+          if (!(ok = mbar_wait_bounded(ds_full, i & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL))) break;
+          tc_fence_after();
+          accumulate(tmem_dK, tmem_Y, q_addr(i), 0, i == 0);
+          accumulate(tmem_dK, tmem_Y, q_addr(i), 1, false);
+          umma_commit(&q_empty[i % BO_QSTAGES]);
+          if (more) {
+            scores(tmem_Y, smem_u32(smem + S::V), o_addr(i + 1), idesc_y);
+            umma_commit(y_full);
+            umma_commit(&o_empty[(i + 1) % BO_OSTAGES]);
           }
         }
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          const uint32_t a_col = (uint32_t)(32 * (kk >> 1) + 8 * (kk & 1));
-          const uint32_t b_off = (uint32_t)(kk * 16 * 128);
-          umma_f16_ts(tmem_A2, tmem_Y + 64 * hb + a_col, make_smem_desc_sw128(c1 + b_off, BW_UNIT_BYTES / 2, 1024), idesc_acc, 1);
-        }
-        umma_commit(&c_empty[st]);
-        return true;
-      };
-      if (ok && par < n_units) {
-        ok = wait_c(par);
-        if (ok) ok = issue_xy(par);
-      }
-      for (uint32_t u = par; u < n_units && ok; u += 2) {
-        // the columns of unit u + 2 are awaited while the compute warps still work on unit u, so
-        // that only the wait for P / dS lies between them and the next MMAs
-        BW_TRACE(1, 1000000 + u);
-        if (u + 2 < n_units) ok = wait_c(u + 2);
-        BW_TRACE(1, 1100000 + u);
-        if (ok) ok = issue_acc(u);
-        BW_TRACE(1, 1300000 + u);
-        if (ok && u + 2 < n_units) ok = issue_xy(u + 2);
-        BW_TRACE(1, 1400000 + u);
       }
       if (ok) umma_commit(acc_full);
     }
-  } else if (warp >= 2) {
+  } else if (warp >= 4) {
     // ----------------------------------------------- compute + epilogue warps
-    // 8 warps: two per TMEM lane quarter; thread (row, hh) owns columns [32·hh, +32) of its row in
-    // every 64-column unit, and columns [64·hh, +64) of the accumulators in the epilogue
+    // two warps per TMEM lane quarter; thread (row, hh): KV slot `row`, columns [32·hh, +32) of both halves
+    // of every query tile, columns [64·hh, +64) of the accumulators (head size 64: [32·hh, +32))
     const int quarter = warp & 3;
-    const int hh = (warp - 2) >> 2;
+    const int hh = (warp - 4) >> 2;
     const int row = quarter * 32 + lane;
-    const int tid = threadIdx.x - 64;  // 0..255
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-    bool ok = n_active > 0;
-    uint32_t s = 0, grp_phase = 0;
-    int tr_n = (warp == 2 && lane == 0) ? 0 : (1 << 30);  // only the first compute warp records
-    auto group_sync = [&]() -> bool {
-      mbar_arrive(grp_bar);
-      const bool done = mbar_wait_bounded(grp_bar, grp_phase, abort_flag, p.status, STATUS_TIMEOUT_MISC);
-      grp_phase ^= 1;
-      return done;
-    };
-    // per-row constants
-    float row_nlse = -INFINITY, row_ndls = 0.f;
-    int row_pos = 0, row_tp = INT_MAX;
-    bool row_valid;
-    int hq = 0, tq = 0;
-    if (MODE == MODE_DQ) {
-      hq = row / p.npos;
-      tq = rt * p.npos + row % p.npos;
-      row_valid = row < p.rows_used && tq < p.T;
-      if (!row_valid) hq = 0;
-      row_pos = p.input_pos + tq;
-      if (row_valid) {
-        const long long idx = ((long long)b * p.H + g * p.gs + hq) * p.T + tq;
-        row_nlse = -p.lse[idx] * 1.4426950408889634f;
-        row_ndls = -p.delta[idx] * p.scale;
-      }
-    } else {
-      const int j = rt * 128 + row;
-      row_valid = j < p.L;
-      if (row_valid) row_tp = p.token_pos ? p.token_pos[b * p.tp_sb + g * p.tp_sg + j] : j;
-    }
-    // MODE_DKV: statistics of query tile ct, column cc <-> (head cc / npos, position cc % npos);
-    // threads 0..127 fetch −lse·log2(e), threads 128..255 fetch −delta·scale
-    auto fetch_stat = [&](int ct) -> float {
-      const int cc = tid & 127;                       // column of the tile: unit cc / 64, column cu of the unit
-      const int cu = cc & 63;
-      const int c_hq = (cc >> 6) * p.u_dh + cu / p.hnpos, c_tq = ct * p.npos_col + (cc >> 6) * p.u_dp + cu % p.hnpos;
-      // columns beyond the unit's heads (padding) and positions beyond the chunk: P = exp2(x − inf) = 0, dS = 0
-      if (ct >= n_col_tiles || cu >= p.cols_used || c_tq >= p.T) return tid < 128 ? -INFINITY : 0.f;
-      const long long idx = ((long long)b * p.H + g * p.gs + c_hq) * p.T + c_tq;
-      return tid < 128 ? -p.lse[idx] * 1.4426950408889634f : -p.delta[idx] * p.scale;
-    };
-    auto store_stat = [&](int buf, float v) {
-      if (tid < 128) stat_nlse[buf * 128 + tid] = v;
-      else stat_ndls[buf * 128 + (tid - 128)] = v;
-    };
-    if (ok) {
-      // zero this thread's 64 columns of the accumulator(s): both MMA issuers only ever accumulate
-      uint32_t z[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) z[i] = 0;
-#pragma unroll
-      for (int c = 0; c < HD / 2; c += 16) {
-        if (MODE == MODE_DKV) tmem_st_32x32b_x16(tmem_A1 + lane_base + (uint32_t)((HD / 2) * hh + c), z);
-        tmem_st_32x32b_x16(tmem_A2 + lane_base + (uint32_t)((HD / 2) * hh + c), z);
-      }
-      if (MODE == MODE_DQ) ok = mbar_wait_bounded(r_full, 0, abort_flag, p.status, STATUS_TIMEOUT_FULL);
-      // MODE_DQ row operands: shared memory -> registers -> TMEM. This thread moves features
-      // [64·hh, +64) of its row: one 128-byte swizzled row of chunk hh = 32 columns of bf16 pairs.
-      if (MODE == MODE_DQ && ok && (HD == 128 || hh == 0)) {
-#pragma unroll
-        for (int op = 0; op < 2; ++op) {
-          const uint8_t* src = smem + (op == 0 ? S::R1 : S::R2) + hh * (BW_TILE_BYTES / 2);
-          uint32_t w[32];
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const uint4 q4 = *reinterpret_cast<const uint4*>(src + sw128_offset(row, u));
-            w[4 * u] = q4.x; w[4 * u + 1] = q4.y; w[4 * u + 2] = q4.z; w[4 * u + 3] = q4.w;
-          }
-          const uint32_t dst = (op == 0 ? tmem_R1 : tmem_R2) + lane_base + (uint32_t)(32 * hh);
-          tmem_st_32x32b_x16(dst, w);
-          tmem_st_32x32b_x16(dst + 16, w + 16);
+    const int j = kt * 128 + row;
+    const bool row_valid = j < p.L;
+    int row_tp = INT_MAX;
+    if (row_valid) row_tp = p.token_pos ? p.token_pos[b * p.tp_sb + g * p.tp_sg + j] : j;
+    const uint32_t xaddr = tmem_X + lane_base + (uint32_t)(32 * hh), yaddr = tmem_Y + lane_base + (uint32_t)(32 * hh);
+    const float2 c2 = make_float2(p.scale_log2, p.scale_log2), sc2 = make_float2(p.scale, p.scale);
+    const bool soft = GEN && p.cap_pre != 0.f;
+    bool ok = true;
+    int tr_n = p.trace && blockIdx.x == 0 && warp == 4 && lane == 0 ? 0 : BO_TRACE_OFF;  // only the first compute warp records
+    uint4* ds_dst = reinterpret_cast<uint4*>(p.ds + (((long long)lbg * p.nT + kt) * p.nq + (q_first - p.q0)) * 16384) + (4 * hh) * 128 + row;
+    for (int i = 0; i < n && ok; ++i, ds_dst += 2048) {
+      const float* nlse = reinterpret_cast<const float*>(smem + S::STAT + (i & 1) * 1024) + 32 * hh;
+      const float* ndls = nlse + 128;
+      const int qpos0 = p.input_pos + (q_first + i) * p.npos;
+      uint32_t hide[2] = {0, 0};
+      bool any_hidden = false;
+      if (GEN && p.window > 0) {  // visible iff 0 <= position of the query − token < window
+        const int th = (int)max(min((long long)row_tp - qpos0, (long long)p.npos), 0LL);
+        const int te = (int)max(min((long long)row_tp + p.window - qpos0, (long long)p.npos), 0LL);
+        any_hidden = __any_sync(0xffffffffu, th > 0 || te < p.npos);
+        if (any_hidden) {
+          hide[0] = bo_hidden(32 * hh, p.npos, th) | ~bo_hidden(32 * hh, p.npos, te);
+          hide[1] = bo_hidden(64 + 32 * hh, p.npos, th) | ~bo_hidden(64 + 32 * hh, p.npos, te);
         }
+      } else if (tmax > qpos0) {  // some slot of the tile is newer than the first query
+        const int th = (int)min((long long)row_tp - qpos0, (long long)p.npos);
+        any_hidden = __any_sync(0xffffffffu, th > 0);
+        if (th >= p.npos) {  // newer than every query of the tile
+          hide[0] = hide[1] = 0xffffffffu;
+        } else if (th > 0) {
+          hide[0] = bo_hidden(32 * hh, p.npos, th);
+          hide[1] = bo_hidden(64 + 32 * hh, p.npos, th);
+        }
+      }
+      if (!(ok = mbar_wait_bounded(&st_full[i & 1], (i >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL))) break;
+      uint32_t xr[64];
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {  // the first half is on its way to dV while the second one is computed
+        if (!(ok = mbar_wait_bounded(&x_full[hf], i & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) break;
+        tc_fence_after();
+        tmem_ld_32x32b_x32(xaddr + (uint32_t)(64 * hf), xr + 32 * hf);
+        tmem_ld_wait();
+        uint32_t pk[16];
+        if (soft) {
+          // capped scores: P for dV is packed here, what stays in registers is P (1 − tanh²), the factor of dS
+#pragma unroll
+          for (int e = 0; e < 32; e += 2) {
+            float pp[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              const float t = bo_tanh(__uint_as_float(xr[32 * hf + e + u]) * p.cap_pre);
+              pp[u] = (hide[hf] & (1u << (e + u))) ? 0.f : bo_exp2(fmaf(t, p.cap_l2, nlse[64 * hf + e + u]));
+              xr[32 * hf + e + u] = __float_as_uint(pp[u] * fmaf(-t, t, 1.f));
+            }
+            pk[e >> 1] = pack_bf16x2(pp[0], pp[1]);
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < 32; e += 4) {
+            const float4 nl = *reinterpret_cast<const float4*>(nlse + 64 * hf + e);
+            uint32_t* x = xr + 32 * hf + e;
+            float2 a = ffma2(make_float2(__uint_as_float(x[0]), __uint_as_float(x[1])), c2, make_float2(nl.x, nl.y));
+            float2 c = ffma2(make_float2(__uint_as_float(x[2]), __uint_as_float(x[3])), c2, make_float2(nl.z, nl.w));
+            a = make_float2(bo_exp2(a.x), bo_exp2(a.y));
+            c = make_float2(bo_exp2(c.x), bo_exp2(c.y));
+            x[0] = __float_as_uint(a.x); x[1] = __float_as_uint(a.y); x[2] = __float_as_uint(c.x); x[3] = __float_as_uint(c.y);
+          }
+          if (any_hidden) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+              if (hide[hf] & (1u << e)) xr[32 * hf + e] = 0;
+          }
+#pragma unroll
+          for (int e = 0; e < 16; ++e) pk[e] = pack_bf16x2(__uint_as_float(xr[32 * hf + 2 * e]), __uint_as_float(xr[32 * hf + 2 * e + 1]));
+        }
+        tmem_st_32x32b_x16(xaddr + (uint32_t)(64 * hf), pk);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_full[hf]);
+        BO_TRACE(2, 2200000 + 2 * i + hf);
+      }
+      if (!ok) break;
+      if (!(ok = mbar_wait_bounded(y_full, i & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) break;
+      tc_fence_after();
+      uint32_t dk_[32];
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        uint32_t yr[32];
+        tmem_ld_32x32b_x32(yaddr + (uint32_t)(64 * hf), yr);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 32; e += 4) {
+          const float4 nd = *reinterpret_cast<const float4*>(ndls + 64 * hf + e);
+          const uint32_t* x = xr + 32 * hf + e;
+          float2 a = ffma2(make_float2(__uint_as_float(yr[e]), __uint_as_float(yr[e + 1])), sc2, make_float2(nd.x, nd.y));
+          float2 c = ffma2(make_float2(__uint_as_float(yr[e + 2]), __uint_as_float(yr[e + 3])), sc2, make_float2(nd.z, nd.w));
+          a = fmul2(make_float2(__uint_as_float(x[0]), __uint_as_float(x[1])), a);
+          c = fmul2(make_float2(__uint_as_float(x[2]), __uint_as_float(x[3])), c);
+          dk_[16 * hf + (e >> 1)] = pack_bf16x2(a.x, a.y);
+          dk_[16 * hf + (e >> 1) + 1] = pack_bf16x2(c.x, c.y);
+        }
+        tmem_st_32x32b_x16(yaddr + (uint32_t)(64 * hf), dk_ + 16 * hf);
       }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0 && ok) mbar_arrive(rows_ready);
+      if (lane == 0) mbar_arrive(ds_full);
+      BO_TRACE(2, 2300000 + 2 * i);
+      // workspace: 8 query rows (16 bytes) of 32 consecutive slots per instruction, 512 contiguous bytes per warp. They hold
+      // the warp ≈ 700 of 3220 cycles a tile (64 B/clk to L2); spread over the exponentials, or done by warps of their own
+      // that read dS back from TMEM, they slow the exponentials down by more (both go through the queue of the LSU).
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        __stcs(ds_dst + (8 * (u >> 2) + (u & 3)) * 128, make_uint4(dk_[4 * u], dk_[4 * u + 1], dk_[4 * u + 2], dk_[4 * u + 3]));
     }
-    int ct = next_active(0);
-    if (MODE == MODE_DKV && ok) {
-      store_stat(0, fetch_stat(ct));
-      ok = group_sync();
-    }
-    const float2 c2 = make_float2(p.scale_log2, p.scale_log2);
-    const float2 sc2 = make_float2(p.scale, p.scale);
-    const int32_t* tpp = p.token_pos ? p.token_pos + b * p.tp_sb + g * p.tp_sg : nullptr;
-    while (ct < n_col_tiles && ok) {
-      const bool msk = masked(ct);
-      const int ct_next = next_active(ct + 1);
-      float stat_next = 0.f;
-      if (MODE == MODE_DKV) stat_next = fetch_stat(ct_next);  // in flight while this tile is processed
-      const int sbuf = s & 1;
-      const int cpos0 = p.input_pos + ct * p.npos_col;  // MODE_DKV: first position of the query tile
-      for (int h = 0; h < 2 && ok; ++h) {
-        const int cc0 = 64 * h + 32 * hh;  // first column of this thread within the 128-column tile
-        // MODE_DQ: lane holds the token position of column cc0 + lane (asked for before the wait)
-        int v_tp = INT_MAX;
-        if (MODE == MODE_DQ && msk) {
-          const int jj = ct * 128 + cc0 + lane;
-          if (jj < p.L) v_tp = tpp ? tpp[jj] : jj;
-        }
-        BW_TRACE(2, 2000000 + 2 * s + h);
-        if (!mbar_wait_bounded(&xy_full[h], s & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
-        BW_TRACE(2, 2100000 + 2 * s + h);
-        tc_fence_after();
-        const uint32_t xaddr = tmem_X + lane_base + (uint32_t)(64 * h + 32 * hh);
-        const uint32_t yaddr = tmem_Y + lane_base + (uint32_t)(64 * h + 32 * hh);
-        uint32_t xr[32], yr[32];
-        tmem_ld_32x32b_x32(xaddr, xr);
-        tmem_ld_32x32b_x32(yaddr, yr);
-        tmem_ld_wait();
-        BW_TRACE(2, 2200000 + 2 * s + h);
-        // bit e of `hide`: column cc0 + e is not visible to this thread's row
-        uint32_t hide = 0;
-        bool win_done = false;
-        if constexpr (GEN) {
-         if (msk && win > 0) {
-          // visible iff 0 <= position of the query − token < window
-          win_done = true;
-          if (MODE == MODE_DQ) {
-            uint32_t nm = __ballot_sync(0xffffffffu, v_tp > qpos_min_of(rt) || v_tp <= qpos_max_of(rt) - win);
-            while (nm) {
-              const int e = __ffs(nm) - 1;
-              nm &= nm - 1;
-              const int d = row_pos - __shfl_sync(0xffffffffu, v_tp, e);
-              hide |= (uint32_t)((uint32_t)d >= (uint32_t)win) << e;
-            }
-          } else {
-            const int upos0 = cpos0 + h * p.u_dp;
-            int pp_ = (32 * hh) % p.hnpos;
-#pragma unroll
-            for (int e = 0; e < 32; ++e) {
-              const int d = upos0 + pp_ - row_tp;
-              hide |= (uint32_t)((uint32_t)d >= (uint32_t)win) << e;
-              pp_ = pp_ + 1 == p.hnpos ? 0 : pp_ + 1;
-            }
-          }
-         }
-        }
-        if (msk && !win_done) {
-          if (MODE == MODE_DQ) {
-            // only columns beyond the first query of the CTA need the per-row comparison
-            // (positions broadcast by shuffle)
-            uint32_t nm = __ballot_sync(0xffffffffu, v_tp > qpos_min_of(rt));
-            while (nm) {
-              const int e = __ffs(nm) - 1;
-              nm &= nm - 1;
-              hide |= (uint32_t)(__shfl_sync(0xffffffffu, v_tp, e) > row_pos) << e;
-            }
-          } else if (__any_sync(0xffffffffu, row_tp > cpos0)) {
-            // column cu of unit h holds position cpos0 + h·hnpos + cu % hnpos (head-major columns)
-            const int upos0 = cpos0 + h * p.u_dp;
-            if ((p.hnpos & (p.hnpos - 1)) == 0) {
-#pragma unroll
-              for (int e = 0; e < 32; ++e) hide |= (uint32_t)(row_tp > upos0 + ((32 * hh + e) & (p.hnpos - 1))) << e;
-            } else {
-              int pp_ = (32 * hh) % p.hnpos;
-#pragma unroll
-              for (int e = 0; e < 32; ++e) {
-                hide |= (uint32_t)(row_tp > upos0 + pp_) << e;
-                pp_ = pp_ + 1 == p.hnpos ? 0 : pp_ + 1;
-              }
-            }
-          }
-        }
-        uint32_t pk[16], dk_[16];
-        if (GEN && p.cap_pre != 0.f) {
-          // capped scores: the raw score goes through tanh, and dS takes the factor 1 − tanh² of the cap
-#pragma unroll
-          for (int e = 0; e < 32; e += 2) {
-            float2 nl, nd;
-            if (MODE == MODE_DQ) {
-              nl = make_float2(row_nlse, row_nlse);
-              nd = make_float2(row_ndls, row_ndls);
-            } else {
-              nl = *reinterpret_cast<const float2*>(stat_nlse + sbuf * 128 + cc0 + e);
-              nd = *reinterpret_cast<const float2*>(stat_ndls + sbuf * 128 + cc0 + e);
-            }
-            const float2 th = make_float2(bw_tanh(__uint_as_float(xr[e]) * p.cap_pre), bw_tanh(__uint_as_float(xr[e + 1]) * p.cap_pre));
-            const float2 xx = ffma2(th, make_float2(p.cap_l2, p.cap_l2), nl);
-            float2 pp = make_float2(bw_exp2(xx.x), bw_exp2(xx.y));
-            if (hide & (1u << e)) pp.x = 0.f;
-            if (hide & (1u << (e + 1))) pp.y = 0.f;
-            float2 tt = ffma2(make_float2(__uint_as_float(yr[e]), __uint_as_float(yr[e + 1])), sc2, nd);
-            tt = fmul2(tt, make_float2(fmaf(-th.x, th.x, 1.f), fmaf(-th.y, th.y, 1.f)));
-            const float2 ds = fmul2(pp, tt);
-            pk[e >> 1] = pack_bf16x2(pp.x, pp.y);
-            dk_[e >> 1] = pack_bf16x2(ds.x, ds.y);
-          }
-        } else
-#pragma unroll
-        for (int e = 0; e < 32; e += 2) {
-          float2 nl, nd;
-          if (MODE == MODE_DQ) {
-            nl = make_float2(row_nlse, row_nlse);
-            nd = make_float2(row_ndls, row_ndls);
-          } else {
-            nl = *reinterpret_cast<const float2*>(stat_nlse + sbuf * 128 + cc0 + e);
-            nd = *reinterpret_cast<const float2*>(stat_ndls + sbuf * 128 + cc0 + e);
-          }
-          const float2 xx = ffma2(make_float2(__uint_as_float(xr[e]), __uint_as_float(xr[e + 1])), c2, nl);
-          float2 pp = make_float2(bw_exp2(xx.x), bw_exp2(xx.y));
-          if (hide & (1u << e)) pp.x = 0.f;
-          if (hide & (1u << (e + 1))) pp.y = 0.f;
-          const float2 tt = ffma2(make_float2(__uint_as_float(yr[e]), __uint_as_float(yr[e + 1])), sc2, nd);
-          const float2 ds = fmul2(pp, tt);
-          pk[e >> 1] = pack_bf16x2(pp.x, pp.y);
-          dk_[e >> 1] = pack_bf16x2(ds.x, ds.y);
-        }
-        BW_TRACE(2, 2300000 + 2 * s + h);
-        // P and dS go back into the first 16 columns of the 32 that this thread has just read
-        if (MODE == MODE_DKV) tmem_st_32x32b_x16(xaddr, pk);
-        tmem_st_32x32b_x16(yaddr, dk_);
-        tmem_st_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&pds_full[h]);
-        BW_TRACE(2, 2400000 + 2 * s + h);
-      }
-      if (!ok) break;
-      if (MODE == MODE_DKV) {
-        // the other buffer was last read during the previous tile, before that tile's barrier
-        store_stat(sbuf ^ 1, stat_next);
-        if (!group_sync()) { ok = false; break; }
-      }
-      ++s;
-      ct = ct_next;
-    }
-    // ---- epilogue
+    // ---- epilogue: fp32 tiles -> padded rows in shared memory (the Q ring is free) -> coalesced vector reductions.
+    // Every address is touched by this CTA only, so the sums do not depend on any order.
     if (ok) ok = mbar_wait_bounded(acc_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL);
     if (ok) {
       tc_fence_after();
-      if (MODE == MODE_DQ) {
-        __nv_bfloat16* dst = p.dq + (((long long)b * p.H + g * p.gs + hq) * p.T + tq) * HD;
+      constexpr int W = HD / 2, LPR = W / 4;  // fp32 of a half row, lanes that add one
+      uint8_t* buf = smem + S::Q + (warp - 4) * 32 * S::ROW;
+      const long long off = b * p.dk_sb + g * p.dk_sg + (long long)(kt * 128 + quarter * 32) * HD + W * hh;
+      const int rows = min(32, p.L - (kt * 128 + quarter * 32));
 #pragma unroll 1
-        for (int c0 = (HD / 2) * hh; c0 < (HD / 2) * (hh + 1); c0 += 32) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(tmem_A2 + lane_base + (uint32_t)c0, r);
-          tmem_ld_wait();
-          if (row_valid) {
+      for (int w = 0; w < 2; ++w) {
+        uint32_t r[W];
+        const uint32_t src = (w == 0 ? tmem_dV : tmem_dK) + lane_base + (uint32_t)(W * hh);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              uint4 o;
-              o.x = pack_bf16x2(__uint_as_float(r[8 * u + 0]), __uint_as_float(r[8 * u + 1]));
-              o.y = pack_bf16x2(__uint_as_float(r[8 * u + 2]), __uint_as_float(r[8 * u + 3]));
-              o.z = pack_bf16x2(__uint_as_float(r[8 * u + 4]), __uint_as_float(r[8 * u + 5]));
-              o.w = pack_bf16x2(__uint_as_float(r[8 * u + 6]), __uint_as_float(r[8 * u + 7]));
-              *reinterpret_cast<uint4*>(dst + c0 + 8 * u) = o;
-            }
-          }
-        }
-      } else {
-        const long long off = b * p.dk_sb + g * p.dk_sg + (long long)(rt * 128 + row) * HD;
-#pragma unroll 1
-        for (int c0 = (HD / 2) * hh; c0 < (HD / 2) * (hh + 1); c0 += 32) {
-          uint32_t r1v[32], r2v[32];
-          tmem_ld_32x32b_x32(tmem_A1 + lane_base + (uint32_t)c0, r1v);
-          tmem_ld_32x32b_x32(tmem_A2 + lane_base + (uint32_t)c0, r2v);
-          tmem_ld_wait();
-          if (row_valid) {
-            // accumulate with vector reductions: no load -> add -> store chain in the epilogue. Every
-            // address is touched by this CTA only, so the result does not depend on any order.
-            float* dvp = p.dv + off + c0;
-            float* dkp = p.dk + off + c0;
+        for (int c = 0; c < W; c += 32) tmem_ld_32x32b_x32(src + (uint32_t)c, r + c);
+        tmem_ld_wait();
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dvp + 4 * u), "f"(__uint_as_float(r1v[4 * u])),
-                           "f"(__uint_as_float(r1v[4 * u + 1])), "f"(__uint_as_float(r1v[4 * u + 2])),
-                           "f"(__uint_as_float(r1v[4 * u + 3]))
-                           : "memory");
-              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dkp + 4 * u), "f"(__uint_as_float(r2v[4 * u])),
-                           "f"(__uint_as_float(r2v[4 * u + 1])), "f"(__uint_as_float(r2v[4 * u + 2])),
-                           "f"(__uint_as_float(r2v[4 * u + 3]))
-                           : "memory");
-            }
-          }
+        for (int u = 0; u < W / 4; ++u)
+          *reinterpret_cast<uint4*>(buf + lane * S::ROW + u * 16) = make_uint4(r[4 * u], r[4 * u + 1], r[4 * u + 2], r[4 * u + 3]);
+        __syncwarp();
+        float* dst = (w == 0 ? p.dv : p.dk) + off + (lane % LPR) * 4;
+#pragma unroll
+        for (int u = 0; u < LPR; ++u) {
+          const int rr = (32 / LPR) * u + lane / LPR;
+          const float4 v = *reinterpret_cast<const float4*>(buf + rr * S::ROW + (lane % LPR) * 16);
+          if (rr < rows)
+            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + rr * HD), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
         }
+        __syncwarp();
       }
-    } else if (n_active == 0 && MODE == MODE_DQ && row_valid) {
-      __nv_bfloat16* dst = p.dq + (((long long)b * p.H + g * p.gs + hq) * p.T + tq) * HD;
-      for (int c = (HD / 2) * hh; c < (HD / 2) * (hh + 1); c += 8) *reinterpret_cast<uint4*>(dst + c) = make_uint4(0, 0, 0, 0);
     }
   }
   tc_fence_before();
@@ -700,6 +538,194 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant_
     tmem_dealloc(tmem_base, 512);
   }
 }
+
+// Descriptor of an MN-major operand without swizzle: core matrices of 8 k-rows x 8 MN elements, 128 contiguous bytes;
+// `k_bytes` / `mn_bytes` lie between core matrices along K (leading offset) and along MN (stride offset).
+__device__ __forceinline__ uint64_t bo_desc_mn(uint32_t smem_addr, uint32_t k_bytes, uint32_t mn_bytes) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_addr >> 4) & 0x3FFF);
+  d |= (uint64_t)((k_bytes >> 4) & 0x3FFF) << 16;
+  d |= (uint64_t)((mn_bytes >> 4) & 0x3FFF) << 32;
+  d |= (uint64_t)1 << 46;
+  return d;
+}
+
+// dQ of one query tile: dS tiles of the workspace (A operand, MN-major without swizzle: element (query row 8u + e, slot r) at
+// 2048·u + 16·r + 2·e, so that the kernel above can write it coalesced) times K tiles (B operand, MN-major).
+// Bound by reading dS: 64 KB per step into shared memory, 512 tensor cycles.
+struct BoDqSmem {
+  static constexpr int RING = 0;  // per stage: dS tile | K tile
+  static constexpr int BAR = RING + BO_QK_STAGES * 2 * BO_TILE;
+  static constexpr int TOTAL = BAR + 128;
+};
+template <bool GEN, int HD>
+__global__ void __launch_bounds__(BO_DQ_THREADS, 1)
+bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const BoParams p) {
+  using S = BoDqSmem;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  if (smem_u32(smem) & 1023u) {
+    if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, STATUS_TIMEOUT_MISC);
+    return;
+  }
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::BAR);
+  uint64_t* full = bars + 0;   // [3]
+  uint64_t* empty = bars + 3;  // [3]
+  uint64_t* acc_full = bars + 6;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 7);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lq = blockIdx.x % p.nq, lbg = blockIdx.x / p.nq;
+  const int qt = p.q0 + lq, bg = p.bg0 + lbg;
+  const int b = bg / p.G, g = bg % p.G;
+  const int32_t* tmin = p.tile_min + (long long)bg * p.nT;
+  const int32_t* tmax = p.tile_max + (long long)bg * p.nT;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < BO_QK_STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(acc_full, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 128);
+    tmem_relinquish();
+  }
+  int n = 0;  // KV tiles that some query of this tile sees: those the kernel above wrote
+  for (int t0 = 0; t0 < p.nT; t0 += BO_DQ_THREADS) {
+    const int t = t0 + (int)threadIdx.x;
+    n += __syncthreads_count(t < p.nT && bo_active<GEN>(p, qt, tmin[t], tmax[t]));
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    uint32_t s = 0;
+    bool ok = true;
+    for (int t0 = 0; t0 < p.nT && ok; t0 += 32) {
+      const int tl = t0 + lane;
+      uint32_t act = __ballot_sync(0xffffffffu, tl < p.nT && bo_active<GEN>(p, qt, tmin[tl], tmax[tl]));
+      while (act && ok) {
+        const int kt = t0 + __ffs(act) - 1;
+        act &= act - 1;
+        const uint32_t st = s % BO_QK_STAGES;
+        if (lane == 0) {
+          ok = mbar_wait_bounded(&empty[st], ((s / BO_QK_STAGES) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_EMPTY);
+          if (ok) {
+            uint8_t* d = smem + S::RING + st * 2 * BO_TILE;
+            mbar_expect_tx(&full[st], BO_TILE + 256 * HD);
+            bulk_load(d, p.ds + (((long long)lbg * p.nT + kt) * p.nq + lq) * 16384, BO_TILE, &full[st]);
+            tma_load_4d(d + BO_TILE, &tmK, &full[st], 0, kt * 128, g, b);
+            if (HD == 128) tma_load_4d(d + BO_TILE + BO_CHUNK, &tmK, &full[st], 64, kt * 128, g, b);
+          }
+        }
+        ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+        ++s;
+      }
+    }
+    if (!ok && lane == 0) {  // let copies in flight land before the CTA's shared memory is released
+      long long c0 = clock64();
+      while (clock64() - c0 < 2000000LL) {
+      }
+    }
+  } else if (warp == 1) {
+    if (n > 0 && elect_one()) {
+      constexpr uint32_t idesc = make_idesc_bf16(128, HD, 1, 1);
+      bool ok = true;
+      int tr_n = p.trace && blockIdx.x == 0 ? 0 : BO_TRACE_OFF;
+      for (int i = 0; i < n && ok; ++i) {
+        const int st = i % BO_QK_STAGES;
+        if (!(ok = mbar_wait_bounded(&full[st], (i / BO_QK_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL))) break;
+        tc_fence_after();
+        const uint32_t a = smem_u32(smem + S::RING + st * 2 * BO_TILE), k = a + BO_TILE;
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)  // 16 slots per step
+          umma_f16_ss(tmem_base, bo_desc_mn(a + (uint32_t)(kk * 256), 128, 2048),
+                      make_smem_desc_sw128(k + (uint32_t)(kk * 16 * 128), BO_CHUNK, 1024), idesc, (i | kk) != 0);
+        umma_commit(&empty[st]);
+        BO_TRACE(1, 1000000 + i);
+      }
+      if (ok) umma_commit(acc_full);
+    }
+  } else {
+    const int quarter = warp & 3;
+    const int row = quarter * 32 + lane;
+    const int hq = row / p.npos, tq = qt * p.npos + row % p.npos;
+    const bool row_valid = row < p.rows_used && tq < p.T;
+    __nv_bfloat16* dst = p.dq + (((long long)b * p.H + g * p.gs + hq) * p.T + tq) * HD;
+    bool ok = true;
+    if (n > 0) ok = mbar_wait_bounded(acc_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL);
+    tc_fence_after();
+    if (ok) {
+#pragma unroll 1
+      for (int c0 = 0; c0 < HD; c0 += 32) {
+        uint32_t r[32];
+        if (n > 0) {
+          tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, r);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) r[e] = 0;
+        }
+        if (row_valid) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            uint4 o;
+            o.x = pack_bf16x2(__uint_as_float(r[8 * u + 0]), __uint_as_float(r[8 * u + 1]));
+            o.y = pack_bf16x2(__uint_as_float(r[8 * u + 2]), __uint_as_float(r[8 * u + 3]));
+            o.z = pack_bf16x2(__uint_as_float(r[8 * u + 4]), __uint_as_float(r[8 * u + 5]));
+            o.w = pack_bf16x2(__uint_as_float(r[8 * u + 6]), __uint_as_float(r[8 * u + 7]));
+            *reinterpret_cast<uint4*>(dst + c0 + 8 * u) = o;
+          }
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 128);
+  }
+}
+
+// Rounds of one call. A round's workspace is pairs · nT · nq tiles of 32 KB; it is kept below 1 GiB, the dS of a chunk of
+// 1024 queries x 32 heads over 16384 slots. Query tiles are divided first: every round then still has all (pair, KV tile)
+// CTAs, so its last wave stays as full as that of one launch. Below 8 query tiles a round would mostly load and store its
+// K, V, dK and dV tiles, and the pairs are divided as well.
+constexpr long long BO_DS_LIMIT = 1LL << 30;
+struct BoRounds {
+  int pairs, nq;
+  BoRounds(long long bg, long long nT, long long nQT) {
+    const long long tiles = BO_DS_LIMIT / BO_TILE;
+    const long long least = nQT < 8 ? nQT : 8;
+    long long pr = tiles / (nT * least);
+    pr = pr < 1 ? 1 : (pr > bg ? bg : pr);
+    long long q = tiles / (nT * pr);
+    q = q < 1 ? 1 : (q > nQT ? nQT : q);
+    const long long n = (nQT + q - 1) / q;
+    pairs = (int)pr;
+    nq = (int)((nQT + n - 1) / n);  // rounds of nearly equal length
+  }
+  long long bytes(long long nT) const { return (long long)pairs * nT * nq * BO_TILE; }
+};
+
+struct BoLayout {  // scratch: tile_min | tile_max | statistics | head-major copy of dO | dS
+  long long stats, dot, ds, total;
+  int npos, nT, nQT;
+  BoRounds rounds;
+  static long long round256(long long n) { return (n + 255) / 256 * 256; }
+  BoLayout(int B, int H, int G, int T, int L)
+      : npos(128 / (H / G)), nT((L + 127) / 128), nQT((T + npos - 1) / npos), rounds((long long)B * G, nT, nQT) {
+    stats = round256(2LL * B * G * nT * 4);
+    dot = stats + (long long)B * G * nQT * 1024;
+    ds = dot + round256((long long)B * H * T * 256);
+    total = ds + rounds.bytes(nT);
+  }
+};
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -725,29 +751,33 @@ static int bw_make_tmap_4d(CUtensorMap* tm, const void* ptr, uint64_t d0, uint64
   return r == CUDA_SUCCESS ? KVB_OK : KVB_ERR_TMAP;
 }
 
-// the two launches of one backward call for one (GEN, head size) instantiation: dQ on the side stream, dK / dV on the caller's
+// all launches of one call for one (GEN, head size) instantiation
 template <bool GEN, int HD>
-static void bw_launch(const CUtensorMap& tmQ, const CUtensorMap& tmdO, const CUtensorMap& tmKh, const CUtensorMap& tmVh,
-                      const BwParams& pq, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmQh,
-                      const CUtensorMap& tmdOh, const BwParams& p, cudaStream_t side, cudaStream_t s) {
+static void bo_launch(const CUtensorMap& tmQ, const CUtensorMap& tmO, const CUtensorMap& tmK, const CUtensorMap& tmV, BoParams p, int BG,
+                      const BoRounds& rounds, long long* trace, int trace_mode, cudaStream_t s) {
   static kvb::PerDeviceOnce attr_once;
   if (attr_once.first()) {
-    cudaFuncSetAttribute(sdpa_bwd_kernel<MODE_DQ, GEN, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwSmem::TOTAL);
-    cudaFuncSetAttribute(sdpa_bwd_kernel<MODE_DKV, GEN, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwSmem::TOTAL);
+    cudaFuncSetAttribute(bwd_dkv_kernel<GEN, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, BoSmem::TOTAL);
+    cudaFuncSetAttribute(bwd_dq_kernel<GEN, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, BoDqSmem::TOTAL);
   }
-  sdpa_bwd_kernel<MODE_DQ, GEN, HD><<<p.B * p.G * p.nQT, BW_THREADS, BwSmem::TOTAL, side>>>(tmQ, tmdO, tmKh, tmVh, pq);
-  sdpa_bwd_kernel<MODE_DKV, GEN, HD><<<p.B * p.G * p.nT, BW_THREADS, BwSmem::TOTAL, s>>>(tmK, tmV, tmQh, tmdOh, p);
+  for (int bg0 = 0; bg0 < BG; bg0 += rounds.pairs) {
+    const int pairs = min(rounds.pairs, BG - bg0);
+    for (int q0 = 0; q0 < p.nQT; q0 += rounds.nq) {
+      p.bg0 = bg0; p.q0 = q0; p.nq = min(rounds.nq, p.nQT - q0);
+      p.trace = trace_mode == 1 ? trace : nullptr;
+      bwd_dkv_kernel<GEN, HD><<<pairs * p.nT, BO_THREADS, BoSmem::TOTAL, s>>>(tmK, tmV, tmQ, tmO, p);
+      p.trace = trace_mode == 0 ? trace : nullptr;
+      bwd_dq_kernel<GEN, HD><<<pairs * p.nq, BO_DQ_THREADS, BoDqSmem::TOTAL, s>>>(tmK, p);
+    }
+  }
 }
 
 }  // namespace kvb
 
-extern "C" int kvb_att_tile_minmax(const int32_t* token_pos, int32_t* tmin, int32_t* tmax, int B, int G, int L, long long tp_sb,
-                                   long long tp_sg, int tile, void* stream);
-
 // Optional timeline trace (diagnostics): `buf` holds 3 roles x `cap` events x 2 int64 (tag, SM clock),
 // filled by CTA 0 of the dQ launch (mode 0) or the dK/dV launch (mode 1) of every later kvb_sdpa_bwd
 // call of this process; buf = NULL switches tracing off. Tags: 1e6+ MMA issuer, 2e6+ compute warp;
-// the digits below 1e5 count 64-column units.
+// the digits below 1e5 count 64-column halves (dK/dV) or KV tiles (dQ).
 static long long* g_bw_trace = nullptr;
 static int g_bw_trace_cap = 0, g_bw_trace_mode = 0;
 extern "C" int kvb_sdpa_bwd_set_trace(void* buf, int cap, int mode) {
@@ -757,11 +787,9 @@ extern "C" int kvb_sdpa_bwd_set_trace(void* buf, int cap, int mode) {
   return KVB_OK;
 }
 
-static long long bw_round4(long long n) { return (n + 3) / 4 * 4; }
-// scratch: tile_min | tile_max (B*G*nT int32 each) | delta (B*H*T fp32) | head-major copy of dO (B*H*T*128 bf16)
 extern "C" long long kvb_sdpa_bwd_scratch_bytes(int B, int H, int G, int q_len, int kv_len) {
-  const long long nT = (kv_len + 127) / 128;
-  return (bw_round4(2LL * B * G * nT) + bw_round4((long long)B * H * q_len)) * 4 + (long long)B * H * q_len * 128 * 2;
+  if (B <= 0 || G <= 0 || q_len <= 0 || kv_len <= 0 || H < G || H / G > 64) return 16;  // refused by the call
+  return kvb::BoLayout(B, H, G, q_len, kv_len).total;
 }
 
 // head_size: 128 or 64; q_sb, q_sh: batch and head strides of q in elements (0, 0: contiguous (B,H,T,D)); window: sliding
@@ -796,93 +824,50 @@ extern "C" int kvb_sdpa_bwd_ex(const void* q, const void* k, const void* v, cons
   if (gs > 64) return KVB_ERR_UNSUPPORTED;  // a 64-column unit of the dK/dV launch holds all heads of a group
   if ((k_sb % 8) || (k_sg % 8) || (dk_sb % 4) || (dk_sg % 4)) return KVB_ERR_ALIGN;
   cudaStream_t s = (cudaStream_t)stream;
-  BwParams p;
-  p.B = B; p.H = H; p.G = G; p.T = q_len; p.L = kv_len;
-  p.gs = gs; p.npos = 128 / gs; p.rows_used = p.npos * gs;
-  if (gs >= 2 && (gs & (gs - 1)) == 0) {  // half of the heads x all positions of the tile per unit
-    p.u_heads = gs / 2; p.u_dh = gs / 2; p.u_dp = 0;
-    p.hnpos = 128 / gs; p.npos_col = p.hnpos;
-  } else {                                 // all heads x half of the positions of the tile per unit
-    p.u_heads = gs; p.u_dh = 0;
-    p.hnpos = 64 / gs; p.u_dp = p.hnpos; p.npos_col = 2 * p.hnpos;
-  }
-  p.cols_used = p.hnpos * p.u_heads;
-  p.nCT = (q_len + p.npos_col - 1) / p.npos_col;
-  p.nT = (kv_len + 127) / 128;
-  p.nQT = (q_len + p.npos - 1) / p.npos;
-  p.token_pos = token_pos; p.tp_sb = tp_sb; p.tp_sg = tp_sg;
-  p.dk_sb = dk_sb; p.dk_sg = dk_sg;
-  int32_t* sc = reinterpret_cast<int32_t*>(scratch);
-  int32_t* tmin = sc;
-  int32_t* tmax = sc + (long long)B * G * p.nT;
-  float* delta = reinterpret_cast<float*>(sc + bw_round4(2LL * B * G * p.nT));
   static const int dout_headmajor = [] {
     const char* e = getenv("KVB200_BWD_DOUT_T");  // "0": read dO in place (diagnostics)
     return (e && e[0] == '0') ? 0 : 1;
   }();
-  __nv_bfloat16* dOt = dout_headmajor ? reinterpret_cast<__nv_bfloat16*>(delta + bw_round4((long long)B * H * q_len)) : nullptr;
-  p.tile_min = tmin; p.tile_max = tmax; p.lse = lse; p.delta = delta;
+  const BoLayout lay(B, H, G, q_len, kv_len);
+  uint8_t* sc = reinterpret_cast<uint8_t*>(scratch);
+  BoParams p;
+  p.G = G; p.H = H; p.T = q_len; p.L = kv_len; p.nT = lay.nT; p.nQT = lay.nQT;
+  p.gs = gs; p.npos = lay.npos; p.rows_used = p.npos * gs;
+  int32_t* tmin = reinterpret_cast<int32_t*>(sc);
+  int32_t* tmax = tmin + (long long)B * G * p.nT;
+  float* stats = reinterpret_cast<float*>(sc + lay.stats);
+  __nv_bfloat16* dOt = reinterpret_cast<__nv_bfloat16*>(sc + lay.dot);
+  p.token_pos = token_pos; p.tile_min = tmin; p.tile_max = tmax; p.stats = stats;
+  p.ds = reinterpret_cast<__nv_bfloat16*>(sc + lay.ds);
   p.dq = (__nv_bfloat16*)dq; p.dk = dk; p.dv = dv;
+  p.tp_sb = tp_sb; p.tp_sg = tp_sg; p.dk_sb = dk_sb; p.dk_sg = dk_sg;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   p.input_pos = input_pos; p.status = status;
+  p.bg0 = p.q0 = p.nq = 0;
   p.window = window;
   p.cap_pre = softcap > 0.f ? scale / softcap : 0.f;
   p.cap_l2 = softcap * 1.4426950408889634f;
+  p.trace = nullptr; p.trace_cap = g_bw_trace_cap;
 
-  // row operands: boxes of npos positions x gs heads (dQ launch) or 128 slots (dK/dV launch); streamed units: boxes of
-  // 64 slots (dQ launch) or hnpos positions x gs heads (dK/dV launch)
-  CUtensorMap tmQ, tmdO, tmK, tmV, tmQh, tmdOh, tmKh, tmVh;
+  // boxes of npos positions x gs heads (Q, dO) or 128 slots (K, V)
+  CUtensorMap tmQ, tmO, tmK, tmV;
   int rc;
-  const uint64_t qT = (uint64_t)q_len, HT = (uint64_t)H * q_len, hd = (uint64_t)head_size;
-  // Q (B,H,T,D): dims (D,T,H,B)
+  const uint64_t hd = (uint64_t)head_size, TD = (uint64_t)q_len * hd, HT = (uint64_t)H * q_len;
   if ((rc = bw_make_tmap_4d(&tmQ, q, hd, q_len, H, B, hd, (uint64_t)q_sh, (uint64_t)q_sb, 64, p.npos, gs))) return rc;
-  if ((rc = bw_make_tmap_4d(&tmQh, q, hd, q_len, H, B, hd, (uint64_t)q_sh, (uint64_t)q_sb, 64, p.hnpos, p.u_heads))) return rc;
-  // dO (B,T,H,D) viewed with dims (D,T,H,B): T stride H*D, H stride D
-  if (dOt) {  // the head-major copy that the delta kernel leaves: same strides as Q
-    if ((rc = bw_make_tmap_4d(&tmdO, dOt, hd, q_len, H, B, hd, qT * hd, HT * hd, 64, p.npos, gs))) return rc;
-    if ((rc = bw_make_tmap_4d(&tmdOh, dOt, hd, q_len, H, B, hd, qT * hd, HT * hd, 64, p.hnpos, p.u_heads))) return rc;
-  } else {
-    if ((rc = bw_make_tmap_4d(&tmdO, dout, hd, q_len, H, B, (uint64_t)H * hd, hd, HT * hd, 64, p.npos, gs))) return rc;
-    if ((rc = bw_make_tmap_4d(&tmdOh, dout, hd, q_len, H, B, (uint64_t)H * hd, hd, HT * hd, 64, p.hnpos, p.u_heads))) return rc;
+  if (dout_headmajor) {  // the head-major copy that the statistics kernel leaves: runs of positions of one head, as for Q
+    if ((rc = bw_make_tmap_4d(&tmO, dOt, hd, q_len, H, B, hd, TD, H * TD, 64, p.npos, gs))) return rc;
+  } else {               // dO (B,T,H,D) viewed with dims (D,T,H,B)
+    if ((rc = bw_make_tmap_4d(&tmO, dout, hd, q_len, H, B, (uint64_t)H * hd, hd, HT * hd, 64, p.npos, gs))) return rc;
   }
   if ((rc = bw_make_tmap_4d(&tmK, k, hd, kv_len, G, B, hd, k_sg, k_sb, 64, 128, 1))) return rc;
   if ((rc = bw_make_tmap_4d(&tmV, v, hd, kv_len, G, B, hd, k_sg, k_sb, 64, 128, 1))) return rc;
-  if ((rc = bw_make_tmap_4d(&tmKh, k, hd, kv_len, G, B, hd, k_sg, k_sb, 64, 64, 1))) return rc;
-  if ((rc = bw_make_tmap_4d(&tmVh, v, hd, kv_len, G, B, hd, k_sg, k_sb, 64, 64, 1))) return rc;
-
-  if ((rc = kvb_att_tile_minmax(token_pos, tmin, tmax, B, G, kv_len, tp_sb, tp_sg, 128, stream))) return rc;
-  const long long rows = (long long)B * q_len * H;
-  if (head_size == 128)
-    att_delta_kernel<128><<<(unsigned)((rows + 7) / 8), 256, 0, s>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, delta, dOt, B, q_len, H);
-  else
-    att_delta_kernel<64><<<(unsigned)((rows + 7) / 8), 256, 0, s>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, delta, dOt, B, q_len, H);
-  // The two launches are independent (dQ | dK, dV). They run on two streams, forked from and joined
-  // back into the caller's stream, so that the tail of one grid (256 CTAs of the dQ launch fill
-  // 148 SMs 1.73 times) is filled with CTAs of the other.
-  static cudaStream_t side[64] = {nullptr};
-  static cudaEvent_t ev_fork[64] = {nullptr}, ev_join[64] = {nullptr};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return KVB_ERR_CUDA;
-  if (!side[dev]) {
-    if (cudaStreamCreateWithFlags(&side[dev], cudaStreamNonBlocking) != cudaSuccess) return KVB_ERR_CUDA;
-    if (cudaEventCreateWithFlags(&ev_fork[dev], cudaEventDisableTiming) != cudaSuccess) return KVB_ERR_CUDA;
-    if (cudaEventCreateWithFlags(&ev_join[dev], cudaEventDisableTiming) != cudaSuccess) return KVB_ERR_CUDA;
-  }
-  cudaEventRecord(ev_fork[dev], s);
-  cudaStreamWaitEvent(side[dev], ev_fork[dev], 0);
-  BwParams pq = p;
-  pq.trace = g_bw_trace_mode == 0 ? g_bw_trace : nullptr; pq.trace_cap = g_bw_trace_cap;
-  p.trace = g_bw_trace_mode == 1 ? g_bw_trace : nullptr; p.trace_cap = g_bw_trace_cap;
-  // the launch with few long CTAs goes first: the short CTAs of the other one fill its second wave
+  if ((rc = kvb_att_tile_minmax(token_pos, tmin, tmax, B, G, kv_len, tp_sb, tp_sg, 128, s))) return rc;
+  const unsigned blocks = (unsigned)((long long)B * G * p.nQT * 16);  // a warp per packed row
+  const __nv_bfloat16 *go = (const __nv_bfloat16*)dout, *o = (const __nv_bfloat16*)out;
+  if (head_size == 128) bo_stats_kernel<128><<<blocks, 256, 0, s>>>(go, o, lse, stats, dOt, B, G, H, q_len, gs, p.npos, p.nQT, scale);
+  else bo_stats_kernel<64><<<blocks, 256, 0, s>>>(go, o, lse, stats, dOt, B, G, H, q_len, gs, p.npos, p.nQT, scale);
   const bool gen = window > 0 || softcap > 0.f;
-  if (head_size == 128) {
-    if (gen) bw_launch<true, 128>(tmQ, tmdO, tmKh, tmVh, pq, tmK, tmV, tmQh, tmdOh, p, side[dev], s);
-    else bw_launch<false, 128>(tmQ, tmdO, tmKh, tmVh, pq, tmK, tmV, tmQh, tmdOh, p, side[dev], s);
-  } else {
-    if (gen) bw_launch<true, 64>(tmQ, tmdO, tmKh, tmVh, pq, tmK, tmV, tmQh, tmdOh, p, side[dev], s);
-    else bw_launch<false, 64>(tmQ, tmdO, tmKh, tmVh, pq, tmK, tmV, tmQh, tmdOh, p, side[dev], s);
-  }
-  cudaEventRecord(ev_join[dev], side[dev]);
-  cudaStreamWaitEvent(s, ev_join[dev], 0);
+  auto launch = head_size == 128 ? (gen ? bo_launch<true, 128> : bo_launch<false, 128>) : (gen ? bo_launch<true, 64> : bo_launch<false, 64>);
+  launch(tmQ, tmO, tmK, tmV, p, B * G, lay.rounds, g_bw_trace, g_bw_trace_mode, s);
   return cudaGetLastError() == cudaSuccess ? KVB_OK : KVB_ERR_LAUNCH;
 }

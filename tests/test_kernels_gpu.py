@@ -410,6 +410,34 @@ def test_sdpa_bwd(B, H, G, T, L, mode):
     assert torch.equal(dk_acc[:, :, L:], dk0[:, :, L:]) and torch.equal(dv_acc[:, :, L:], dv0[:, :, L:])
 
 
+@pytest.mark.parametrize("B,H,G,T,L,mode,window,D", [
+    (1, 1, 1, 1, 1, "arange", None, 128), (1, 64, 1, 5, 130, "perm", None, 128), (1, 2, 2, 129, 257, "arange", None, 64),
+    (1, 8, 2, 500, 500, "arange", 40, 128),        # windows: KV tiles that no query tile sees after, or before, some
+    (1, 32, 8, 2048, 16384, "perm", None, 128),    # 2 GiB of dS: two rounds over the query tiles
+    (5, 8, 8, 1000, 16384, "arange", None, 64)])   # 40 pairs x 8 query tiles x 128 KV tiles: rounds over the pairs
+def test_sdpa_bwd_edges_and_rounds(B, H, G, T, L, mode, window, D):
+    """Smallest and ragged tiles, tile ranges cut by a window, and calls whose dS workspace is filled in rounds."""
+    q = torch.randn(B, H, T, D, device=DEV, dtype=torch.bfloat16)
+    k = torch.randn(B, G, L, D, device=DEV, dtype=torch.bfloat16)
+    v = torch.randn(B, G, L, D, device=DEV, dtype=torch.bfloat16)
+    go = torch.randn(B, T, H * D, device=DEV, dtype=torch.bfloat16)
+    tp, input_pos = None, L - T
+    if mode == "perm":
+        input_pos = 3 * L
+        tp = torch.rand(B, G, L, device=DEV).argsort(dim=-1).to(torch.int32)
+        tp = torch.where(tp >= L - T, tp - (L - T) + input_pos, tp)
+    scale = 1.0 / math.sqrt(D)
+    out, _, lse = _cuda().sdpa_fwd(q, k, v, scale, input_pos, tp, False, window)
+    got = _cuda().sdpa_bwd(go, q, k, v, out, lse, scale, input_pos, tp, sliding_window=window)
+    _cuda().check_status(DEV)
+    for b in range(B):  # one sequence after the other: the reference holds fp32 scores
+        want = ref.sdpa_backward(go[b:b + 1], q[b:b + 1], k[b:b + 1], v[b:b + 1], scale, input_pos, None if tp is None else tp[b:b + 1], window)
+        for a, r in zip(got, want):
+            # P and dS are rounded to bf16 (2^-9 relative, independent per term): 2e-3 of the norm; a lost tile or round is of
+            # order 1. With one visible token dP − δ cancels and dQ, dK are zero up to the rounding of O: 2^-8 per feature
+            assert _rel_err(a[b:b + 1], r) < 1e-2 or (a[b].float() - r[0].float()).norm() < 1e-2 * math.sqrt(r.numel())
+
+
 @pytest.mark.parametrize("B,H,G,T,L,mode,window,softcap", [
     (1, 8, 2, 256, 2048, "perm", None, None), (2, 8, 2, 100, 1000, "perm", None, None), (1, 14, 2, 77, 900, "arange", None, None),
     (1, 32, 8, 700, 700, "arange", None, None), (1, 3, 1, 50, 200, "perm", None, None), (1, 8, 2, 300, 1500, "arange", 256, 3.0)])
