@@ -1210,22 +1210,29 @@ flash256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 }
 
 // ------------------------------------------------------------------ column sums
+// Four warpgroups, each with an S^T buffer and every fourth query tile: with two (two warps per scheduler) the kernel issued
+// in 46 % of the cycles, waiting on its own loads and exponentials. 1024 queries x 32 heads over 16384 slots: 227 us with two
+// warpgroups and normalisers from global memory, 165 with four and normalisers brought by the producer, 151 with the column
+// loop rolled (the unrolled one, twice for masks, missed the instruction cache).
 constexpr int CS_SBUF = 4;
-// K tile | ring of query tiles (four, or two of the 64 KB tiles of head size 256) | barriers | exchange
+constexpr int CS_THREADS = 64 + CS_SBUF * 128;
+constexpr int CS_LSLOTS = 16;  // normalisers of the query tiles (512 B each)
+// K tile | ring of query tiles (four, or two of the 64 KB tiles of head size 256) | normalisers | barriers | exchange
 template <int HD>
 struct CsSmemT {
   static constexpr int TILE = F2_T * (HD < 128 ? 128 : HD) * 2;  // head size 64 keeps the 32 KB slots of 128
   static constexpr int QSTAGES = HD == 256 ? 2 : 4;
   static constexpr int K = 0;
   static constexpr int Q = K + TILE;
-  static constexpr int BAR = Q + QSTAGES * TILE;
-  static constexpr int XCH = BAR + 256;   // 128 floats: sums of the second warpgroup
-  static constexpr int TOTAL = XCH + 512;
+  static constexpr int LSE = Q + QSTAGES * TILE;
+  static constexpr int BAR = LSE + CS_LSLOTS * 512;
+  static constexpr int XCH = BAR + 512;   // 128 floats each: sums of the warpgroups after the first
+  static constexpr int TOTAL = XCH + (CS_SBUF - 1) * 512;
 };
 static_assert(CsSmemT<256>::TOTAL <= 232448, "shared memory of the column-sum kernel exceeds the limit of a CTA");
 
 template <bool GEN, int HD>
-__global__ void __launch_bounds__(F2_THREADS, 1)
+__global__ void __launch_bounds__(CS_THREADS, 1)
 colsum_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const F2Params p) {
   using CsSmem = CsSmemT<HD>;
   constexpr int CS_QSTAGES = CsSmem::QSTAGES;
@@ -1242,7 +1249,8 @@ colsum_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   uint64_t* q_empty = bars + 5;    // [4]
   uint64_t* s_full = bars + 9;     // [4]
   uint64_t* s_empty = bars + 13;   // [4]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
+  uint64_t* l_full = bars + 17;    // [16]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17 + CS_LSLOTS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1271,7 +1279,7 @@ colsum_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 
   if (p.rows_used < F2_T) {
     for (int s = 0; s < CS_QSTAGES; ++s)
-      f2_zero_unused_rows(smem + CsSmem::Q + s * CS_TILE, p.rows_used, threadIdx.x, F2_THREADS, HD / 64);
+      f2_zero_unused_rows(smem + CsSmem::Q + s * CS_TILE, p.rows_used, threadIdx.x, CS_THREADS, HD / 64);
     fence_proxy_async_smem();
   }
   if (threadIdx.x == 0) {
@@ -1284,6 +1292,7 @@ colsum_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       mbar_init(&s_full[s], 1);
       mbar_init(&s_empty[s], 4);
     }
+    for (int s = 0; s < CS_LSLOTS; ++s) mbar_init(&l_full[s], 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -1317,6 +1326,11 @@ colsum_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 #pragma unroll
         for (int cch = 0; cch < HD / 64; ++cch)
           tma_load_4d(qd + cch * F2_CHUNK_BYTES, &tmQ, &q_full[st], 64 * cch, g * p.gs, (qt_first + i) * p.npos, b);
+        // The slot was last read for tile i − 16. The MMAs of tile i − 4 were complete for this stage to be free, so the
+        // buffer of tile i − 8 had been handed back, by a warpgroup that was done with i − 12 and with i − 16 before.
+        const int ls = i % CS_LSLOTS;
+        mbar_expect_tx(&l_full[ls], 512);
+        bulk_load(smem + CsSmem::LSE + ls * 512, p.lse2 + (bg * p.nQT + (qt_first + i)) * F2_T, 512, &l_full[ls]);
       }
       if (!ok) {
         long long c0 = clock64();
@@ -1325,7 +1339,7 @@ colsum_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && n_q > 0) {
+    if (n_q > 0 && elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(F2_T, F2_T, 0, 0);  // K (slots = M) and Q (rows = N), both K-major
       bool ok = mbar_wait_bounded(k_full, 0, abort_flag, p.status, STATUS_TIMEOUT_FULL);
       const uint32_t k_addr = smem_u32(smem + CsSmem::K);
@@ -1351,84 +1365,70 @@ colsum_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     const int slot_in_tile = quarter * 32 + lane;   // TMEM lane = slot of the tile
     const int j = t * F2_T + slot_in_tile;
     const int pj = p.pos[(bg * p.nT + t) * F2_T + slot_in_tile];
-    const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+    const uint32_t tS = tmem_base + (uint32_t)(wg * F2_T) + ((uint32_t)(quarter * 32) << 16);
     const float c = p.scale_log2;
     const float2 c2 = make_float2(c, c);
-    float2 acc0 = make_float2(0.f, 0.f), acc1 = acc0;
+    float total = 0.f;
     bool ok = true;
-    auto lse_row = [&](int i) { return p.lse2 + (bg * p.nQT + (qt_first + i)) * F2_T; };
-    auto prefetch_lse = [&](int i) {  // 512 bytes = four lines, one per 8 lanes is enough: lanes 0..3 ask
-      if (i < n_q && lane < 4) asm volatile("prefetch.global.L1 [%0];" ::"l"(lse_row(i) + 32 * lane));
-    };
-    prefetch_lse(wg);
-    for (int i = wg; i < n_q && ok; i += 2) {
+    for (int i = wg; i < n_q && ok; i += CS_SBUF) {
       const int qt = qt_first + i;
-      const int sb = i % CS_SBUF;
-      prefetch_lse(i + 2);
       // row e of the query tile sits at position qt·npos + e / gs: the slot is visible from column thr on
       const long long first_vis = ((long long)pj - p.input_pos - (long long)qt * p.npos) * p.gs;
       const int thr = first_vis <= 0 ? 0 : (first_vis >= F2_T ? F2_T : (int)first_vis);
       // with a window the slot is visible up to (not including) column thr_hi
       const long long end_vis = first_vis + (long long)c_window * p.gs;
       const int thr_hi = c_window <= 0 ? F2_T : (end_vis <= 0 ? 0 : (end_vis >= F2_T ? F2_T : (int)end_vis));
-      const bool masked = __any_sync(0xffffffffu, thr > 0 || thr_hi < F2_T);
-      const float4* lp = reinterpret_cast<const float4*>(lse_row(i));
-      if (!mbar_wait_bounded(&s_full[sb], (i / CS_SBUF) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) {
-        ok = false;
-        break;
-      }
+      // A slot that no row of the tile sees drops the sum of the tile; only where some row sees it and some does not (one
+      // tile in the life of a new token) are the columns looked at one by one.
+      const bool none = thr >= thr_hi;
+      const bool masked = __any_sync(0xffffffffu, !none && (thr > 0 || thr_hi < F2_T));
+      const int ls = i % CS_LSLOTS;
+      const float4* lp = reinterpret_cast<const float4*>(smem + CsSmem::LSE + ls * 512);
+      if (!(ok = mbar_wait_bounded(&l_full[ls], (i / CS_LSLOTS) & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL))) break;
+      if (!(ok = mbar_wait_bounded(&s_full[wg], (i / CS_SBUF) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) break;
       tc_fence_after();
-      // 32 columns at a time: the next chunk of scores and of normalisers travels while this one is summed
-      const uint32_t tS = tmem_base + (uint32_t)(sb * F2_T) + lane_base;
-      uint32_t x[2][32];
-      float4 ls[2][8];
-      tmem_ld_32x32b_x32(tS, x[0]);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) ls[0][k] = __ldg(lp + k);
-#pragma unroll
+      // 32 columns at a time in a rolled loop: the other warps of the scheduler cover the load, and the code stays in the
+      // instruction cache
+      float2 acc0 = make_float2(0.f, 0.f), acc1 = acc0;
+#pragma unroll 1
       for (int u = 0; u < 4; ++u) {
+        uint32_t x[32];
+        tmem_ld_32x32b_x32(tS + (uint32_t)(32 * u), x);
         tmem_ld_wait();
-        if (u < 3) {
-          tmem_ld_32x32b_x32(tS + (uint32_t)(32 * (u + 1)), x[(u + 1) & 1]);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) ls[(u + 1) & 1][k] = __ldg(lp + 8 * (u + 1) + k);
-        } else {
-          // the whole tile has left TMEM: hand the buffer back before the last chunk is summed
+        if (u == 3) {  // the whole tile has left TMEM: hand the buffer back before the last chunk is summed
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&s_empty[sb]);
+          if (lane == 0) mbar_arrive(&s_empty[wg]);
+        }
+        if (soft) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) x[e] = __float_as_uint(f2_softcap(__uint_as_float(x[e]), p.cap_pre, p.cap_post));
+        }
+        if (masked) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (32 * u + e < thr || 32 * u + e >= thr_hi) x[e] = 0xff800000u;
         }
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          const int e = 32 * u + 4 * k;
-          const float4 lv = ls[u & 1][k];
-          float2 r0 = make_float2(__uint_as_float(x[u & 1][4 * k]), __uint_as_float(x[u & 1][4 * k + 1]));
-          float2 r1 = make_float2(__uint_as_float(x[u & 1][4 * k + 2]), __uint_as_float(x[u & 1][4 * k + 3]));
-          if (soft) {
-            r0 = make_float2(f2_softcap(r0.x, p.cap_pre, p.cap_post), f2_softcap(r0.y, p.cap_pre, p.cap_post));
-            r1 = make_float2(f2_softcap(r1.x, p.cap_pre, p.cap_post), f2_softcap(r1.y, p.cap_pre, p.cap_post));
-          }
-          const float2 x0 = ffma2(r0, c2, make_float2(-lv.x, -lv.y));
-          const float2 x1 = ffma2(r1, c2, make_float2(-lv.z, -lv.w));
-          float2 y0 = cs_pair_on_fma(2 * k) ? f2_exp2_poly2(x0) : make_float2(f2_exp2(x0.x), f2_exp2(x0.y));
-          float2 y1 = cs_pair_on_fma(2 * k + 1) ? f2_exp2_poly2(x1) : make_float2(f2_exp2(x1.x), f2_exp2(x1.y));
-          if (masked) {
-            if (e < thr || e >= thr_hi) y0.x = 0.f;
-            if (e + 1 < thr || e + 1 >= thr_hi) y0.y = 0.f;
-            if (e + 2 < thr || e + 2 >= thr_hi) y1.x = 0.f;
-            if (e + 3 < thr || e + 3 >= thr_hi) y1.y = 0.f;
-          }
-          acc0 = fadd2(acc0, y0);
-          acc1 = fadd2(acc1, y1);
+          const float4 lv = lp[8 * u + k];
+          const float2 x0 = ffma2(make_float2(__uint_as_float(x[4 * k]), __uint_as_float(x[4 * k + 1])), c2, make_float2(-lv.x, -lv.y));
+          const float2 x1 = ffma2(make_float2(__uint_as_float(x[4 * k + 2]), __uint_as_float(x[4 * k + 3])), c2, make_float2(-lv.z, -lv.w));
+          acc0 = fadd2(acc0, cs_pair_on_fma(2 * k) ? f2_exp2_poly2(x0) : make_float2(f2_exp2(x0.x), f2_exp2(x0.y)));
+          acc1 = fadd2(acc1, cs_pair_on_fma(2 * k + 1) ? f2_exp2_poly2(x1) : make_float2(f2_exp2(x1.x), f2_exp2(x1.y)));
         }
       }
+      if (!none) total += (acc0.x + acc0.y) + (acc1.x + acc1.y);
     }
-    // the two warpgroups hold the even and the odd query tiles of the same slots: add them in a fixed order
+    // the warpgroups hold every fourth query tile of the same slots each: add them in a fixed order
     float* xch = reinterpret_cast<float*>(smem + CsSmem::XCH);
-    const float mine = (acc0.x + acc0.y) + (acc1.x + acc1.y);
-    if (wg == 1) xch[slot_in_tile] = mine;
-    asm volatile("bar.sync 1, 256;" ::: "memory");
-    if (wg == 0 && j < p.L && p.weights) p.weights[bg * p.L + j] = ok ? (mine + xch[slot_in_tile]) * p.inv_gs : 0.f;
+    if (wg > 0) xch[(wg - 1) * F2_T + slot_in_tile] = total;
+    asm volatile("bar.sync 1, 512;" ::: "memory");
+    if (wg == 0 && j < p.L && p.weights) {
+#pragma unroll
+      for (int w = 0; w < CS_SBUF - 1; ++w) total += xch[w * F2_T + slot_in_tile];
+      p.weights[bg * p.L + j] = ok ? total * p.inv_gs : 0.f;
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -1479,7 +1479,7 @@ static int f2_launch(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUten
     const long long rows = (long long)p.B * p.G * p.nQT * F2_T;
     flash_merge_kernel<HD><<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(p);
   }
-  if (p.weights) colsum_kernel<GEN, HD><<<p.B * p.G * p.nT, F2_THREADS, CsSmemT<HD>::TOTAL, s>>>(tmQ, tmK, p);
+  if (p.weights) colsum_kernel<GEN, HD><<<p.B * p.G * p.nT, CS_THREADS, CsSmemT<HD>::TOTAL, s>>>(tmQ, tmK, p);
   return cudaGetLastError() == cudaSuccess ? KVB_OK : KVB_ERR_LAUNCH;
 }
 
@@ -1498,8 +1498,8 @@ static int f3_launch(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUten
     flash_merge_kernel<256><<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(p);
   }
   if (p.weights) {
-    if (gen) colsum_kernel<true, 256><<<p.B * p.G * p.nT, F2_THREADS, CsSmemT<256>::TOTAL, s>>>(tmQ, tmK, p);
-    else colsum_kernel<false, 256><<<p.B * p.G * p.nT, F2_THREADS, CsSmemT<256>::TOTAL, s>>>(tmQ, tmK, p);
+    if (gen) colsum_kernel<true, 256><<<p.B * p.G * p.nT, CS_THREADS, CsSmemT<256>::TOTAL, s>>>(tmQ, tmK, p);
+    else colsum_kernel<false, 256><<<p.B * p.G * p.nT, CS_THREADS, CsSmemT<256>::TOTAL, s>>>(tmQ, tmK, p);
   }
   return cudaGetLastError() == cudaSuccess ? KVB_OK : KVB_ERR_LAUNCH;
 }
