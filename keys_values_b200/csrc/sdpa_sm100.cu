@@ -243,11 +243,8 @@ __device__ __forceinline__ float2 f2_exp2_poly2(float2 x) {
   r.y = __int_as_float(__float_as_int(q.y) + (__float_as_int(t.y) << 23));
   return r;
 }
-// of every 8 pairs of scores, the pairs listed here take the FMA-pipe exponential
-// (none in the flash kernel: once the softmax warps were off the critical path, the tensor-core side bounded it
-// and the extra FMA-pipe instructions cost more than the shorter exponential phase gained)
-__device__ __forceinline__ constexpr bool f2_pair_on_fma(int pair) { return false && pair < 0; }
-// the column-sum kernel is bound by the exponentials alone: 3 of 8 pairs go to the FMA pipe
+// The column-sum kernel is bound by the exponentials alone: 3 of 8 pairs go to the FMA pipe. None do in the flash kernel, where
+// the tensor side bounds a step and the extra FMA-pipe instructions cost more than the shorter exponential phase gained.
 __device__ __forceinline__ constexpr bool cs_pair_on_fma(int pair) { return (pair & 7) == 0 || (pair & 7) == 3 || (pair & 7) == 6; }
 
 // Rows of a query tile that TMA does not write (npos · gs < 128) are cleared once, so that their
@@ -280,9 +277,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint64_t* kv_full = bars + 2;    // [4]
   uint64_t* kv_empty = bars + 6;   // [4]
   uint64_t* s_full = bars + 10;    // [2]
-  uint64_t* p_full = bars + 12;    // [2]
-  uint64_t* o_full = bars + 14;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  uint64_t* p_full = bars + 12;    // [2 query tiles][2 halves of 64 slots]
+  uint64_t* o_full = bars + 16;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   uint8_t* tflags = smem + F2Smem::TF;
 
@@ -332,7 +329,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     for (int i = 0; i < 2; ++i) {
       mbar_init(&q_full[i], 1);
       mbar_init(&s_full[i], 1);
-      mbar_init(&p_full[i], 4);
+      mbar_init(&p_full[2 * i], 4);
+      mbar_init(&p_full[2 * i + 1], 4);
     }
     for (int s = 0; s < F2_STAGES; ++s) {
       mbar_init(&kv_full[s], 1);
@@ -425,7 +423,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------- MMA issuer
-    if (lane == 0 && n_active > 0) {
+    if (n_active > 0 && elect_one()) {
       constexpr uint32_t idesc_qk = make_idesc_bf16(F2_T, F2_T, 0, 0);  // Q, K both K-major
       constexpr uint32_t idesc_pv = make_idesc_bf16(F2_T, HD, 0, 1);    // P K-major (TMEM), V MN-major
       bool ok = true;
@@ -460,10 +458,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         ++t_next;
         return m;
       };
-      auto issue_pv = [&](int w, uint32_t vseq, bool first) {
+      auto issue_pv = [&](int w, uint32_t vseq, int h, bool first) {  // slots [64·h, +64) of the tile
         const uint32_t v_addr = stage_addr(vseq);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
+        for (int kk = 4 * h; kk < 4 * h + 4; ++kk) {
           // A = P from TMEM: 16 slots = 8 columns of packed bf16 pairs per step.
           // B = V: MN-major; 16 slot rows per step (2048 B); the two 64-wide feature chunks are LBO apart.
           umma_f16_ts(tmem_base + (uint32_t)(2 * F2_T + w * F2_T), tmem_base + (uint32_t)(w * F2_T + 8 * kk),
@@ -491,10 +489,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const bool m_next = more ? next_active_masked() : false;
         for (int w = 0; w < 2 && ok; ++w) {
           F2_MARK(6);
-          if (!(ok = mbar_wait_bounded(&p_full[w], i & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL))) break;
+          if (!(ok = mbar_wait_bounded(&p_full[2 * w], i & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL))) break;
+          tc_fence_after();
+          issue_pv(w, vseq, 0, i == 0);
+          if (!(ok = mbar_wait_bounded(&p_full[2 * w + 1], i & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL))) break;
           F2_MARK(2 * w);
           tc_fence_after();
-          issue_pv(w, vseq, i == 0);
+          issue_pv(w, vseq, 1, false);
           if (w == 1) umma_commit(&kv_empty[vseq % F2_STAGES]);
           if (more) {
             issue_qk(w, knext, m_next);
@@ -699,8 +700,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           for (int e = 0; e < 32; e += 4) {
             const float2 x0 = ffma2(make_float2(__uint_as_float(x[u & 1][e]), __uint_as_float(x[u & 1][e + 1])), c2, neg_m2);
             const float2 x1 = ffma2(make_float2(__uint_as_float(x[u & 1][e + 2]), __uint_as_float(x[u & 1][e + 3])), c2, neg_m2);
-            const float2 y0 = f2_pair_on_fma(e >> 1) ? f2_exp2_poly2(x0) : make_float2(f2_exp2(x0.x), f2_exp2(x0.y));
-            const float2 y1 = f2_pair_on_fma((e >> 1) + 1) ? f2_exp2_poly2(x1) : make_float2(f2_exp2(x1.x), f2_exp2(x1.y));
+            const float2 y0 = make_float2(f2_exp2(x0.x), f2_exp2(x0.y));
+            const float2 y1 = make_float2(f2_exp2(x1.x), f2_exp2(x1.y));
             s0 = fadd2(s0, y0);
             s1 = fadd2(s1, y1);
             pk[e >> 1] = pack_bf16x2(y0.x, y0.y);
@@ -709,6 +710,12 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           // the load of chunk u + 1 (columns 32(u+1) ..) must have left TMEM before P of chunk u lands on
           // columns 16u .. 16u+15 only if those overlap, which they never do (16u + 16 <= 32(u + 1))
           tmem_st_32x32b_x16(tmem_S + (uint32_t)(16 * u), pk);
+          if (u == 1) {  // PV of the first 64 slots runs while the second half is computed
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&p_full[2 * wg]);
+          }
         }
       }
       s0 = fadd2(s0, s1);
@@ -717,7 +724,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[wg]);
+      if (lane == 0) mbar_arrive(&p_full[2 * wg + 1]);
       F2_MARK(5);
       ++i;
     }
@@ -972,7 +979,7 @@ flash256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------- MMA issuer
-    if (lane == 0 && n_active > 0) {
+    if (n_active > 0 && elect_one()) {
       constexpr uint32_t idesc_qk = make_idesc_bf16(F2_T, F2_T, 0, 0);    // Q, K both K-major
       constexpr uint32_t idesc_pv = make_idesc_bf16(F2_T, F3_HD, 0, 1);   // P K-major (TMEM), V MN-major, N = 256
       const uint32_t q_addr = smem_u32(smem + F3Smem::Q), k_addr = smem_u32(smem + F3Smem::K), v_addr = smem_u32(smem + F3Smem::V);
