@@ -88,6 +88,26 @@ struct F2Smem {
 };
 static_assert(F2Smem::TOTAL <= 232448, "shared memory of the flash kernel exceeds the limit of a CTA");
 
+// The unit of a CTA and the KV tiles that it takes: all of them, or the range of its split.
+struct F2Unit {
+  int unit, split, t_lo, t_hi;
+  bool part;
+  template <typename P>
+  __device__ __forceinline__ explicit F2Unit(const P& p) {
+    const int k = (int)blockIdx.x - p.n_full;
+    part = k >= 0;
+    unit = part ? p.n_full + k / p.n_split : (int)blockIdx.x;
+    split = part ? k % p.n_split : 0;
+    t_lo = part ? split * p.tiles_per_split : 0;
+    t_hi = part ? min(p.nT, t_lo + p.tiles_per_split) : p.nT;
+  }
+  // row `row` of the unit (of `rows`) in the partial buffers
+  template <typename P>
+  __device__ __forceinline__ long long part_row(const P& p, int rows, int row) const {
+    return ((long long)(unit - p.n_full) * p.n_split + split) * rows + row;
+  }
+};
+
 struct F2Params {
   const int32_t* pos;        // (B,G,nT*128) padded token positions (INT_MAX beyond the cache)
   const int32_t* tile_min;   // (B,G,nT)
@@ -102,11 +122,12 @@ struct F2Params {
   int input_pos;
   int* status;
   long long* trace;          // optional phase profile of CTA 0: 4 roles x 8 cycle counters
-  // split over the KV axis (few query tiles): grid.y = n_split CTAs per query-tile pair, each over tiles_per_split KV
-  // tiles; they write normalised fp32 partial outputs and their log2 normalisers, a merge kernel combines them
-  int n_split, tiles_per_split;
-  float* part_o;             // (n_split, B, H, T, D)
-  float* part_lse2;          // (n_split, B, H, T), -inf for a split that saw no visible slot
+  // Units (query-tile pairs; single tiles at head size 256) in the order of the grid: the first n_full have one CTA each, the
+  // others n_split CTAs, each over tiles_per_split KV tiles. Those write normalised fp32 partial outputs and their log2
+  // normalisers, which a merge kernel combines.
+  int n_full, n_split, tiles_per_split;
+  float* part_o;             // (units − n_full, n_split, rows of a unit, D)
+  float* part_lse2;          // (units − n_full, n_split, rows of a unit), -inf for a split that saw no visible slot
   // Sliding window (0: none): a slot is visible to a query at position q iff q - window < token <= q.
   // Logit soft-capping (cap_pre = 0: none): the score scale·s becomes cap·tanh(scale·s / cap); the kernels rewrite the
   // raw score s as cap_post·tanh(cap_pre·s) with cap_pre = scale / cap, cap_post = cap / scale and go on as without.
@@ -285,9 +306,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nPair = (p.nQT + 1) / 2;
-  const int pair = blockIdx.x % nPair;
-  const int g = (blockIdx.x / nPair) % p.G;
-  const int b = blockIdx.x / (nPair * p.G);
+  const F2Unit un(p);
+  const int pair = un.unit % nPair;
+  const int g = (un.unit / nPair) % p.G;
+  const int b = un.unit / (nPair * p.G);
   const int t0 = 2 * pair * p.npos;  // first position of the pair
   const int qpos_min = p.input_pos + t0;
   const int qpos_max = p.input_pos + min(t0 + 2 * p.npos, p.T) - 1;
@@ -295,10 +317,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int32_t* tmin = p.tile_min + bg * p.nT;
   const int32_t* tmax = p.tile_max + bg * p.nT;
 
-  // the KV tiles of this CTA: all of them, or the range of its split (tiles outside count as inactive)
-  const int split = p.n_split > 1 ? (int)blockIdx.y : 0;
-  const int t_lo = p.n_split > 1 ? split * p.tiles_per_split : 0;
-  const int t_hi = p.n_split > 1 ? min(p.nT, t_lo + p.tiles_per_split) : p.nT;
+  // tiles outside the range of a split count as inactive
   // With a window, tokens at or below lo_all are hidden from every row of the CTA, those at or below lo_some from some row.
   const int f_window = GEN ? p.window : 0;
   const int lo_all = f_window > 0 ? qpos_min - f_window : INT_MIN;
@@ -306,13 +325,19 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const bool soft = GEN && p.cap_pre != 0.f;
   constexpr bool general = GEN;  // masked tiles are then always treated element by element
   auto calc_bits = [&](int t) -> uint32_t {
-    if (t < t_lo || t >= t_hi) return 0u;
+    if (t < un.t_lo || t >= un.t_hi) return 0u;
     const int lo = tmin[t], hi = tmax[t];
     const uint32_t act = (lo <= qpos_max) && (hi > lo_all);
     const uint32_t msk = (hi > qpos_min) || (lo <= lo_some) || soft;  // soft-capping rewrites every tile
     return act | (msk << 1);
   };
-  for (int t = threadIdx.x; t < min(p.nT, F2_MAX_FLAG_TILES); t += F2_THREADS) tflags[t] = (uint8_t)calc_bits(t);
+  int n_active = 0;
+  for (int t0_ = 0; t0_ < p.nT; t0_ += F2_THREADS) {
+    const int t = t0_ + (int)threadIdx.x;
+    const uint32_t bits = t < p.nT ? calc_bits(t) : 0u;
+    if (t < min(p.nT, F2_MAX_FLAG_TILES)) tflags[t] = (uint8_t)bits;
+    n_active += __syncthreads_count(bits & 1u);
+  }
   auto tile_bits = [&](int t) -> uint32_t { return t >= F2_MAX_FLAG_TILES ? calc_bits(t) : (uint32_t)tflags[t]; };
   if (p.rows_used < F2_T) {
     f2_zero_unused_rows(smem + F2Smem::Q, p.rows_used, threadIdx.x, F2_THREADS, HD / 64);
@@ -349,8 +374,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   // columns: S0 [0,128) | S1 [128,256) | O0 [256,384) | O1 [384,512); P aliases the first 64 columns of its S
-  int n_active = 0;
-  for (int t = 0; t < p.nT; ++t) n_active += (int)(tile_bits(t) & 1u);
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -374,11 +397,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       F2_TRACE_DECL(lane == 0);
       int4 pv_next = make_int4(0, 0, 0, 0);
       {
-        int tf = 0;
-        while (tf < p.nT && !(tile_bits(tf) & 1u)) ++tf;
-        if (tf < p.nT && (tile_bits(tf) & 2u)) pv_next = __ldg(reinterpret_cast<const int4*>(pos_row + (long long)tf * F2_T) + lane);
+        int tf = un.t_lo;
+        while (tf < un.t_hi && !(tile_bits(tf) & 1u)) ++tf;
+        if (tf < un.t_hi && (tile_bits(tf) & 2u)) pv_next = __ldg(reinterpret_cast<const int4*>(pos_row + (long long)tf * F2_T) + lane);
       }
-      for (int t = 0; t < p.nT && ok; ++t) {
+      for (int t = un.t_lo; t < un.t_hi && ok; ++t) {
         const uint32_t tb = tile_bits(t);
         if (!(tb & 1u)) continue;
         for (int kv = 0; kv < 2 && ok; ++kv) {
@@ -387,8 +410,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           if (kv == 0) {
             // positions of the next active tile travel while this one is handled
             int tn = t + 1;
-            while (tn < p.nT && !(tile_bits(tn) & 1u)) ++tn;
-            if (tn < p.nT && (tile_bits(tn) & 2u)) pv_next = __ldg(reinterpret_cast<const int4*>(pos_row + (long long)tn * F2_T) + lane);
+            while (tn < un.t_hi && !(tile_bits(tn) & 1u)) ++tn;
+            if (tn < un.t_hi && (tile_bits(tn) & 2u)) pv_next = __ldg(reinterpret_cast<const int4*>(pos_row + (long long)tn * F2_T) + lane);
           }
           F2_MARK(2);
           ok = mbar_wait_bounded(&kv_empty[st], ((seq / F2_STAGES) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_EMPTY);
@@ -451,10 +474,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         umma_commit(&s_full[w]);
       };
       // the issuer walks the active tiles in step with the producer
-      int t_next = 0;
+      int t_next = un.t_lo;
       auto next_active_masked = [&]() -> bool {
-        while (t_next < p.nT && !(tile_bits(t_next) & 1u)) ++t_next;
-        const bool m = t_next < p.nT && (tile_bits(t_next) & 2u);
+        while (t_next < un.t_hi && !(tile_bits(t_next) & 1u)) ++t_next;
+        const bool m = t_next < un.t_hi && (tile_bits(t_next) & 2u);
         ++t_next;
         return m;
       };
@@ -541,7 +564,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     };
     auto next_active = [&](int t) {
       int tn = t + 1;
-      while (tn < p.nT && !(tile_bits(tn) & 1u)) ++tn;
+      while (tn < un.t_hi && !(tile_bits(tn) & 1u)) ++tn;
       return tn;
     };
     bool ok = n_active > 0;
@@ -549,10 +572,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     int i = 0;
     F2_TRACE_DECL((warp == 2 || warp == 6) && lane == 0);  // the first warp of each warpgroup records
     {
-      const int tf = next_active(-1);
-      if (ok && tf < p.nT && (tile_bits(tf) & 2u)) request_positions(tf);
+      const int tf = next_active(un.t_lo - 1);
+      if (ok && tf < un.t_hi && (tile_bits(tf) & 2u)) request_positions(tf);
     }
-    for (int t = 0; t < p.nT && ok; ++t) {
+    for (int t = un.t_lo; t < un.t_hi && ok; ++t) {
       const uint32_t tb = tile_bits(t);
       if (!(tb & 1u)) continue;
       // Masks. Slots beyond the last query of the CTA arrive as -inf from the MMA. What is left are slots
@@ -577,7 +600,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
       {
         const int tn = next_active(t);
-        if (tn < p.nT && (tile_bits(tn) & 2u)) request_positions(tn);
+        if (tn < un.t_hi && (tile_bits(tn) & 2u)) request_positions(tn);
       }
       F2_MARK(6);
       if (!mbar_wait_bounded(&s_full[wg], i & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) {
@@ -736,9 +759,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tc_fence_after();
       const float inv_l = l > 0.f ? 1.f / l : 0.f;
       const float lse2 = l > 0.f ? m_used + log2f(l) : INFINITY;
-      if (p.n_split > 1) {
+      if (un.part) {
         // partial result of this split: normalised fp32 rows and their log2 normaliser
-        const long long prow = (((long long)split * p.B + b) * p.H + (g * p.gs + (row_valid ? hq : 0))) * p.T + (row_valid ? tq : 0);
+        const long long prow = un.part_row(p, 2 * F2_T, wg * F2_T + row);
         float* pdst = p.part_o + prow * HD;
 #pragma unroll 1
         for (int c0 = 0; c0 < HD; c0 += 32) {
@@ -798,16 +821,22 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 }
 
 // Combines the partial results of the splits of a query row: out = Σ_s w_s O_s / Σ_s w_s with w_s = 2^(lse2_s − max),
-// in a fixed order of the splits. One warp per packed query row (the rows of the lse2 layout, padding rows included,
-// which get +inf there as in the unsplit kernel); lane l holds features 4l .. 4l+3.
+// in a fixed order of the splits. One warp per packed query row of the divided units (padding rows included, which get
+// +inf in the lse2 layout as in the unsplit kernel); lane s first holds the normaliser of split s (n_split <= 32), then lane l
+// the features PER·l .. PER·l + PER − 1. The loads of the splits do not wait for one another.
 template <int HD>
 __global__ void __launch_bounds__(256) flash_merge_kernel(const F2Params p) {
-  const long long wrow = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);  // index into (B, G, nQT, 128)
+  constexpr int TILES = HD == 256 ? 1 : 2;  // query tiles of a unit
+  const int nU = (p.nQT + TILES - 1) / TILES;
+  const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);  // row among those of the divided units
   const int lane = threadIdx.x & 31;
-  if (wrow >= (long long)p.B * p.G * p.nQT * F2_T) return;
-  const int row = (int)(wrow % F2_T);
-  const int qt = (int)((wrow / F2_T) % p.nQT);
-  const long long bg = wrow / ((long long)F2_T * p.nQT);
+  const long long unit = p.n_full + r / (TILES * F2_T);
+  if (unit >= (long long)p.B * p.G * nU) return;
+  const int urow = (int)(r % (TILES * F2_T)), row = urow % F2_T;
+  const int qt = TILES * (int)(unit % nU) + urow / F2_T;
+  if (qt >= p.nQT) return;
+  const long long bg = unit / nU;
+  const long long wrow = (bg * p.nQT + qt) * F2_T + row;  // index into (B, G, nQT, 128)
   const int g = (int)(bg % p.G), b = (int)(bg / p.G);
   const int pl = row / p.gs, hq = row % p.gs;
   const int tq = qt * p.npos + pl;
@@ -817,28 +846,24 @@ __global__ void __launch_bounds__(256) flash_merge_kernel(const F2Params p) {
     return;
   }
   const int h = g * p.gs + hq;
-  const long long stride = (long long)p.B * p.H * p.T;  // rows per split
-  const long long prow = ((long long)b * p.H + h) * p.T + tq;
-  float mx = -INFINITY;
-  for (int sidx = 0; sidx < p.n_split; ++sidx) mx = fmaxf(mx, p.part_lse2[sidx * stride + prow]);
-  constexpr int PER = HD / 32;  // features per lane: lane l holds features PER·l .. PER·l + PER − 1
+  const long long prow = (unit - p.n_full) * p.n_split * (TILES * F2_T) + urow;
+  const float lse_s = lane < p.n_split ? p.part_lse2[prow + (long long)lane * (TILES * F2_T)] : -INFINITY;
+  const float mx = warp_max(lse_s);
+  const float w_s = lse_s > -INFINITY ? exp2f(lse_s - mx) : 0.f;
+  const float total = warp_sum(w_s);
+  constexpr int PER = HD / 32;
   float acc[PER];
 #pragma unroll
   for (int e = 0; e < PER; ++e) acc[e] = 0.f;
-  float total = 0.f;
-  if (mx > -INFINITY) {
-    for (int sidx = 0; sidx < p.n_split; ++sidx) {
-      const float w = exp2f(p.part_lse2[sidx * stride + prow] - mx);
-      if (w > 0.f) {
-        const float2* src = reinterpret_cast<const float2*>(p.part_o + (sidx * stride + prow) * HD + PER * lane);
+#pragma unroll 4
+  for (int sidx = 0; sidx < p.n_split; ++sidx) {
+    const float w = __shfl_sync(0xffffffffu, w_s, sidx);
+    const float2* src = reinterpret_cast<const float2*>(p.part_o + (prow + (long long)sidx * (TILES * F2_T)) * HD + PER * lane);
 #pragma unroll
-        for (int e = 0; e < PER / 2; ++e) {
-          const float2 o = src[e];
-          acc[2 * e] += w * o.x;
-          acc[2 * e + 1] += w * o.y;
-        }
-        total += w;
-      }
+    for (int e = 0; e < PER / 2; ++e) {
+      const float2 o = src[e];
+      acc[2 * e] += w * o.x;
+      acc[2 * e + 1] += w * o.y;
     }
   }
   const float inv = total > 0.f ? 1.f / total : 0.f;
@@ -847,7 +872,7 @@ __global__ void __launch_bounds__(256) flash_merge_kernel(const F2Params p) {
   for (int e = 0; e < PER / 2; ++e) dst[e] = pack_bf16x2(acc[2 * e] * inv, acc[2 * e + 1] * inv);
   if (lane == 0) {
     const float lse2 = total > 0.f ? mx + log2f(total) : INFINITY;
-    if (p.lse) p.lse[prow] = lse2 * 0.6931471805599453f;
+    if (p.lse) p.lse[((long long)b * p.H + h) * p.T + tq] = lse2 * 0.6931471805599453f;
     if (p.lse2) p.lse2[wrow] = lse2;
   }
 }
@@ -898,29 +923,33 @@ flash256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint8_t* tflags = smem + F3Smem::TF;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qt = blockIdx.x % p.nQT;
-  const int g = (blockIdx.x / p.nQT) % p.G;
-  const int b = blockIdx.x / (p.nQT * p.G);
+  const F2Unit un(p);
+  const int qt = un.unit % p.nQT;
+  const int g = (un.unit / p.nQT) % p.G;
+  const int b = un.unit / (p.nQT * p.G);
   const int t0 = qt * p.npos;
   const int qpos_min = p.input_pos + t0;
   const int qpos_max = p.input_pos + min(t0 + p.npos, p.T) - 1;
   const long long bg = (long long)b * p.G + g;
   const int32_t* tmin = p.tile_min + bg * p.nT;
   const int32_t* tmax = p.tile_max + bg * p.nT;
-  const int split = p.n_split > 1 ? (int)blockIdx.y : 0;
-  const int t_lo = p.n_split > 1 ? split * p.tiles_per_split : 0;
-  const int t_hi = p.n_split > 1 ? min(p.nT, t_lo + p.tiles_per_split) : p.nT;
   const int lo_all = p.window > 0 ? qpos_min - p.window : INT_MIN;   // tokens at or below: outside every row's window
   const int lo_some = p.window > 0 ? qpos_max - p.window : INT_MIN;  // ... outside some row's window
   const bool soft = p.cap_pre != 0.f;
   auto calc_bits = [&](int t) -> uint32_t {
-    if (t < t_lo || t >= t_hi) return 0u;
+    if (t < un.t_lo || t >= un.t_hi) return 0u;
     const int lo = tmin[t], hi = tmax[t];
     const uint32_t act = (lo <= qpos_max) && (hi > lo_all);
     const uint32_t msk = (hi > qpos_min) || (lo <= lo_some) || soft;
     return act | (msk << 1);
   };
-  for (int t = threadIdx.x; t < min(p.nT, F2_MAX_FLAG_TILES); t += F3_THREADS) tflags[t] = (uint8_t)calc_bits(t);
+  int n_active = 0;
+  for (int t0_ = 0; t0_ < p.nT; t0_ += F3_THREADS) {
+    const int t = t0_ + (int)threadIdx.x;
+    const uint32_t bits = t < p.nT ? calc_bits(t) : 0u;
+    if (t < min(p.nT, F2_MAX_FLAG_TILES)) tflags[t] = (uint8_t)bits;
+    n_active += __syncthreads_count(bits & 1u);
+  }
   auto tile_bits = [&](int t) -> uint32_t { return t >= F2_MAX_FLAG_TILES ? calc_bits(t) : (uint32_t)tflags[t]; };
   if (p.rows_used < F2_T) {
     f2_zero_unused_rows(smem + F3Smem::Q, p.rows_used, threadIdx.x, F3_THREADS, F3_HD / 64);
@@ -948,8 +977,6 @@ flash256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  int n_active = 0;
-  for (int t = 0; t < p.nT; ++t) n_active += (int)(tile_bits(t) & 1u);
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -961,7 +988,7 @@ flash256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       for (int c = 0; c < 4; ++c) tma_load_4d(smem + F3Smem::Q + c * F2_CHUNK_BYTES, &tmQ, q_full, 64 * c, g * p.gs, t0, b);
       bool ok = true;
       int i = 0;
-      for (int t = 0; t < p.nT && ok; ++t) {
+      for (int t = un.t_lo; t < un.t_hi && ok; ++t) {
         if (!(tile_bits(t) & 1u)) continue;
         if (!(ok = mbar_wait_bounded(k_empty, (i & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_EMPTY))) break;
         mbar_expect_tx(k_full, F3_TILE_BYTES);
@@ -1037,7 +1064,7 @@ flash256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     bool ok = n_active > 0;
     float m_used = -1e30f, l = 0.f;
     int i = 0;
-    for (int t = 0; t < p.nT && ok; ++t) {
+    for (int t = un.t_lo; t < un.t_hi && ok; ++t) {
       const uint32_t tb = tile_bits(t);
       if (!(tb & 1u)) continue;
       const uint32_t tmem_S = tmem_base + (uint32_t)((i & 1) * F2_T) + lane_base;
@@ -1157,8 +1184,8 @@ flash256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       const float lse2 = l > 0.f ? m_used + log2f(l) : INFINITY;
       const int h = g * p.gs + (row_valid ? hq : 0);
       const int tqv = row_valid ? tq : 0;
-      if (p.n_split > 1) {
-        const long long prow = (((long long)split * p.B + b) * p.H + h) * p.T + tqv;
+      if (un.part) {
+        const long long prow = un.part_row(p, F2_T, row);
         float* pdst = p.part_o + prow * F3_HD;
 #pragma unroll 1
         for (int c0 = 0; c0 < F3_HD; c0 += 32) {
@@ -1480,12 +1507,9 @@ static int f2_launch(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUten
     cudaFuncSetAttribute(flash_fwd_kernel<GEN, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, F2Smem::TOTAL);
     cudaFuncSetAttribute(colsum_kernel<GEN, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, CsSmemT<HD>::TOTAL);
   }
-  const int nPair = (p.nQT + 1) / 2;
-  flash_fwd_kernel<GEN, HD><<<dim3(p.B * p.G * nPair, p.n_split), F2_THREADS, F2Smem::TOTAL, s>>>(tmQ, tmK, tmV, p);
-  if (p.n_split > 1) {
-    const long long rows = (long long)p.B * p.G * p.nQT * F2_T;
-    flash_merge_kernel<HD><<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(p);
-  }
+  const int divided = p.B * p.G * ((p.nQT + 1) / 2) - p.n_full;
+  flash_fwd_kernel<GEN, HD><<<p.n_full + divided * p.n_split, F2_THREADS, F2Smem::TOTAL, s>>>(tmQ, tmK, tmV, p);
+  if (divided > 0) flash_merge_kernel<HD><<<divided * (2 * F2_T / 8), 256, 0, s>>>(p);
   if (p.weights) colsum_kernel<GEN, HD><<<p.B * p.G * p.nT, CS_THREADS, CsSmemT<HD>::TOTAL, s>>>(tmQ, tmK, p);
   return cudaGetLastError() == cudaSuccess ? KVB_OK : KVB_ERR_LAUNCH;
 }
@@ -1499,11 +1523,9 @@ static int f3_launch(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUten
     cudaFuncSetAttribute(colsum_kernel<false, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, CsSmemT<256>::TOTAL);
     cudaFuncSetAttribute(colsum_kernel<true, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, CsSmemT<256>::TOTAL);
   }
-  flash256_fwd_kernel<<<dim3(p.B * p.G * p.nQT, p.n_split), F3_THREADS, F3Smem::TOTAL, s>>>(tmQ, tmK, tmV, p);
-  if (p.n_split > 1) {
-    const long long rows = (long long)p.B * p.G * p.nQT * F2_T;
-    flash_merge_kernel<256><<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(p);
-  }
+  const int divided = p.B * p.G * p.nQT - p.n_full;
+  flash256_fwd_kernel<<<p.n_full + divided * p.n_split, F3_THREADS, F3Smem::TOTAL, s>>>(tmQ, tmK, tmV, p);
+  if (divided > 0) flash_merge_kernel<256><<<divided * (F2_T / 8), 256, 0, s>>>(p);
   if (p.weights) {
     if (gen) colsum_kernel<true, 256><<<p.B * p.G * p.nT, CS_THREADS, CsSmemT<256>::TOTAL, s>>>(tmQ, tmK, p);
     else colsum_kernel<false, 256><<<p.B * p.G * p.nT, CS_THREADS, CsSmemT<256>::TOTAL, s>>>(tmQ, tmK, p);
@@ -1535,22 +1557,32 @@ extern "C" int kvb_sdpa_fwd_set_trace(void* buf) {
 
 // Scratch layout (int32 words, 16-byte aligned parts), provided by the caller:
 //   tile_min (B*G*nT) | tile_max (B*G*nT) | positions (B*G*nT*128) | lse2 (B*G*nQT*128 floats)
-// Number of CTAs along the KV axis per query-tile pair: 1 unless the launch would leave most SMs idle (few queries:
-// short chunks at batch 1) while the cache is long enough to give every split at least 8 tiles.
-static int f2_num_splits(long long ctas, long long nT) {
-  static const int enabled = [] {
-    const char* e = getenv("KVB200_F2_SPLIT");  // "0" switches the split off (diagnostics)
-    return (e && e[0] == '0') ? 0 : 1;
-  }();
-  if (!enabled || ctas <= 0 || ctas * 2 > 148 || nT < 16) return 1;
-  long long n = 148 / ctas;
-  if (n > nT / 8) n = nT / 8;
-  if (n > 8) n = 8;
-  return n < 2 ? 1 : (int)n;
-}
+// Units of a launch that are divided over the KV axis: those of a last wave that would leave half of the SMs or more idle,
+// when the cache is long enough. Whole waves stay undivided (no partial results to write and merge), the rest gets as many
+// CTAs as there are SMs, of at least 4 KV tiles each (a CTA's start, its partial results and their merge cost about two).
+// 2 x 499 queries x 40 heads over 7919 slots (160 units): the 12 of the second wave as 12 x 12 CTAs, flash 315 -> 189 us,
+// the call 446 -> 329.
+struct F2Split {
+  long long n_full;
+  int n_split;
+  F2Split(long long units, long long nT) : n_full(units), n_split(1) {
+    static const int enabled = [] {
+      const char* e = getenv("KVB200_F2_SPLIT");  // "0" switches the split off (diagnostics)
+      return (e && e[0] == '0') ? 0 : 1;
+    }();
+    const long long rest = units > 0 ? units % 148 : 0;
+    if (!enabled || rest == 0 || rest * 2 > 148 || nT < 16) return;
+    long long n = 148 / rest;
+    if (n > nT / 4) n = nT / 4;
+    if (n > 16) n = 16;
+    if (n < 2) return;
+    n_full = units - rest;
+    n_split = (int)n;
+  }
+  long long part_rows(long long units, int rows) const { return (units - n_full) * n_split * rows; }
+};
 
-//   ... | split partials: part_lse2 (n_split*B*H*T floats) | part_o (n_split*B*H*T*128 floats), present when the
-//   launch is split over the KV axis (f2_num_splits)
+//   ... | partial results of the divided units: part_lse2 (a float per row) | part_o (a row of floats each)
 extern "C" long long kvb_sdpa_fwd_scratch_bytes(int B, int H, int G, int q_len, int kv_len) {
   if (G <= 0 || H % G || H / G > 128) return -1;
   const int gs = H / G;
@@ -1559,10 +1591,11 @@ extern "C" long long kvb_sdpa_fwd_scratch_bytes(int B, int H, int G, int q_len, 
   const long long nQT = (q_len + npos - 1) / npos;
   const long long bgt = kvb::f2_round4((long long)B * G * nT);
   long long words = 2 * bgt + (long long)B * G * nT * 128 + (long long)B * G * nQT * 128;
-  const int n_split = f2_num_splits((long long)B * G * ((nQT + 1) / 2), nT);
-  // partial outputs sized for the largest head size (256); the number of splits of a launch never exceeds this one's
-  if (n_split > 1) words += kvb::f2_round4((long long)n_split * B * H * q_len) + (long long)n_split * B * H * q_len * 256;
-  return words * 4;
+  // pairs of query tiles (head size 64, 128) or single ones (256), whichever needs more
+  const long long pairs = (long long)B * G * ((nQT + 1) / 2), tiles = (long long)B * G * nQT;
+  const long long r2 = F2Split(pairs, nT).part_rows(pairs, 256), r3 = F2Split(tiles, nT).part_rows(tiles, 128);
+  const long long w2 = kvb::f2_round4(r2) + r2 * 128, w3 = kvb::f2_round4(r3) + r3 * 256;
+  return (words + (w2 > w3 ? w2 : w3)) * 4;
 }
 
 // q (B,H,T,128) contiguous bf16; k, v (B,G,L,128) bf16 with batch / group strides k_sb, k_sg (elements);
@@ -1635,10 +1668,12 @@ extern "C" int kvb_sdpa_fwd_ex(const void* q, const void* k, const void* v, cons
 
   f2_prepare_kernel<<<B * G * p.nT, F2_T, 0, s>>>(token_pos, tmin, tmax, pos, G, kv_len, p.nT, tp_sb, tp_sg);
   const int nPair = head_size == 256 ? p.nQT : (p.nQT + 1) / 2;  // head size 256: one query tile per CTA
-  p.n_split = f2_num_splits((long long)B * G * nPair, p.nT);
+  const F2Split split((long long)B * G * nPair, p.nT);
+  p.n_full = (int)split.n_full;
+  p.n_split = split.n_split;
   p.tiles_per_split = (p.nT + p.n_split - 1) / p.n_split;
   p.part_lse2 = lse2 + (long long)B * G * p.nQT * 128;
-  p.part_o = p.part_lse2 + f2_round4((long long)p.n_split * B * H * q_len);
+  p.part_o = p.part_lse2 + f2_round4(split.part_rows((long long)B * G * nPair, head_size == 256 ? 128 : 256));
   const bool gen = window > 0 || softcap > 0.f;
   if (head_size == 256) return f3_launch(tmQ, tmK, tmV, p, gen, s);
   if (head_size == 128) return gen ? f2_launch<true, 128>(tmQ, tmK, tmV, p, s) : f2_launch<false, 128>(tmQ, tmK, tmV, p, s);

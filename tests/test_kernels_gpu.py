@@ -311,6 +311,15 @@ def test_sdpa_head_size_64(B, H, G, T, L, mode, window, softcap):
     _sdpa_case(B, H, G, T, L, 3 * L if mode == "perm" else L - T, mode, window=window, softcap=softcap, D=64)
 
 
+@pytest.mark.parametrize("B,H,G,T,L,mode,D", [
+    (2, 40, 8, 499, 2100, "perm", 128),   # 160 units: one whole wave, 12 of the next divided by 4 (17 KV tiles)
+    (1, 32, 8, 1209, 2500, "arange", 64),  # 152 units
+    (2, 8, 4, 1211, 2500, "perm", 256),    # 152 units of one query tile
+    (1, 4, 1, 33, 8100, "arange", 128)])   # one unit in 15 parts (64 KV tiles, the last part short)
+def test_sdpa_divides_only_the_last_wave(B, H, G, T, L, mode, D):
+    _sdpa_case(B, H, G, T, L, 3 * L if mode == "perm" else L - T, mode, D=D)
+
+
 @pytest.mark.parametrize("D", [128, 64])
 def test_sdpa_reads_a_slice_of_positions_in_place(D):
     """The queries of a chunk are a slice of the cell's (B,H,T',D) tensor: forward and backward read it through the
