@@ -39,6 +39,11 @@ namespace kvb {
 constexpr int BO_TILE = 128 * 128 * 2;       // 32 KB: two 64-feature chunks of [128 rows x 128 B]
 constexpr int BO_CHUNK = BO_TILE / 2;
 constexpr int BO_QSTAGES = 3, BO_OSTAGES = 2;  // Q lives from S(i) to dK(i), dO from dP(i) to dV(i)
+// Barriers of "thread A has issued S(i + 1)", used in turn. Nothing that A needs for tile i + 1 hangs on B having looked at the
+// one of tile i (P(i + 1) comes after dS(i), whose dP(i) B issued a tile before), so a single barrier could move on by two
+// phases and B would miss its own. Arrival i + 2 needs P(i + 2), hence dS(i + 1) and dP(i + 1), which B issues after its wait
+// for tile i: two barriers are enough.
+constexpr int BO_TURNS = 2;
 constexpr int BO_THREADS = 384;              // producer, issuer A, issuer B, idle, 8 compute warps
 constexpr int BO_QK_STAGES = 3;              // dq kernel: dS tile | K tile per stage
 constexpr int BO_DQ_THREADS = 192;           // producer, issuer, 4 epilogue warps
@@ -198,8 +203,8 @@ bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
   uint64_t* y_full = bars + 18;
   uint64_t* ds_full = bars + 19;
   uint64_t* acc_full = bars + 20;  // one commit per issuer
-  uint64_t* a_issued = bars + 21;  // thread A has issued S(i + 1)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
+  uint64_t* a_issued = bars + 21;  // [BO_TURNS] thread A has issued S(i + 1)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21 + BO_TURNS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -241,7 +246,7 @@ bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
     mbar_init(y_full, 1);
     mbar_init(ds_full, 8);
     mbar_init(acc_full, 2);
-    mbar_init(a_issued, 1);
+    for (int u = 0; u < BO_TURNS; ++u) mbar_init(&a_issued[u], 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -346,7 +351,7 @@ bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
             BO_TRACE(1, 1200000 + 2 * i + h);
           }
           if (!ok) break;
-          mbar_arrive(a_issued);
+          mbar_arrive(&a_issued[i % BO_TURNS]);
         }
       } else {
         ok = mbar_wait_bounded(v_full, 0, abort_flag, p.status, STATUS_TIMEOUT_FULL) && wait_o(0);
@@ -360,7 +365,7 @@ bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
           const bool more = i + 1 < n;
           if (!(ok = wait_q(i) && (!more || wait_o(i + 1)))) break;
           // The next scores go first: the exponentials hang on them, and the tensor pipe serves both threads in turn.
-          if (!(ok = mbar_wait_bounded(a_issued, i & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL))) break;
+          if (!(ok = mbar_wait_bounded(&a_issued[i % BO_TURNS], (i / BO_TURNS) & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL))) break;
           if (!(ok = mbar_wait_bounded(ds_full, i & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL))) break;
           tc_fence_after();
           accumulate(tmem_dK, tmem_Y, q_addr(i), 0, i == 0);
