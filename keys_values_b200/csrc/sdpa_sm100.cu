@@ -84,7 +84,8 @@ struct F2Smem {
   static constexpr int QX = TF + F2_MAX_FLAG_TILES;             // [128 x 16] bf16, column 0 = 1: A operand of the bias step
   static constexpr int KX = QX + F2_BIAS_TILE_BYTES;            // per ring stage: [128 x 16] bf16, column 0 = 0 or -inf
   static constexpr int BAR = KX + F2_STAGES * F2_BIAS_TILE_BYTES;
-  static constexpr int TOTAL = BAR + 256;
+  static constexpr int TR = BAR + 256;  // diagnostics: 4 roles x (8 counters, clock of the last mark)
+  static constexpr int TOTAL = TR + 160;
 };
 static_assert(F2Smem::TOTAL <= 232448, "shared memory of the flash kernel exceeds the limit of a CTA");
 
@@ -122,9 +123,9 @@ struct F2Params {
   int input_pos;
   int* status;
   long long* trace;          // optional phase profile of CTA 0: 4 roles x 8 cycle counters
-  // Units (query-tile pairs; single tiles at head size 256) in the order of the grid: the first n_full have one CTA each, the
-  // others n_split CTAs, each over tiles_per_split KV tiles. Those write normalised fp32 partial outputs and their log2
-  // normalisers, which a merge kernel combines.
+  // Units (query-tile pairs; single tiles at head size 256) in the order of the grid, numbered (group, tile, sequence): the first
+  // n_full, as many of every sequence, have one CTA each, the others n_split CTAs, each over tiles_per_split KV tiles. Those
+  // write normalised fp32 partial outputs and their log2 normalisers, which a merge kernel combines.
   int n_full, n_split, tiles_per_split;
   float* part_o;             // (units − n_full, n_split, rows of a unit, D)
   float* part_lse2;          // (units − n_full, n_split, rows of a unit), -inf for a split that saw no visible slot
@@ -148,20 +149,28 @@ __device__ __forceinline__ float f2_softcap(float s, float pre, float post) {
 }
 
 // Optional phase profile of CTA 0 (diagnostics): each role adds the cycles spent since its previous mark to one of
-// eight counters and writes them once at the end, so that the measurement costs a clock read per mark.
+// eight counters and writes them once at the end, so that the measurement costs a clock read per mark. The counters lie in
+// shared memory: the loops of the flash kernel have no registers for them (1024 queries x 32 heads over 16384 slots: 468 us with
+// the counters in registers, 464 so).
 // Roles: 0 MMA issuer, 1 / 2 first warp of softmax warpgroup 0 / 1, 3 producer.
 __device__ __forceinline__ uint32_t f2_clock() {
   uint32_t c;
   asm volatile("mov.u32 %0, %%clock;" : "=r"(c));
   return c;
 }
-#define F2_TRACE_DECL(active) uint32_t tr_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}; const bool tr_on = p.trace != nullptr && blockIdx.x == 0 && (active); uint32_t tr_last = tr_on ? f2_clock() : 0u
+#define F2_TRACE_DECL(role, active)                                                                    \
+  uint32_t* const tr_acc = reinterpret_cast<uint32_t*>(smem + F2Smem::TR) + 9 * (role);                \
+  const bool tr_on = p.trace != nullptr && blockIdx.x == 0 && (active);                                \
+  if (tr_on) {                                                                                         \
+    for (int k_ = 0; k_ < 8; ++k_) tr_acc[k_] = 0;                                                     \
+    tr_acc[8] = f2_clock();                                                                            \
+  }
 #define F2_MARK(k)                                \
   do {                                            \
     if (tr_on) {                                  \
       const uint32_t now_ = f2_clock();           \
-      tr_acc[k] += now_ - tr_last;                \
-      tr_last = now_;                             \
+      tr_acc[k] += now_ - tr_acc[8];              \
+      tr_acc[8] = now_;                           \
     }                                             \
   } while (0)
 #define F2_TRACE_STORE(role)                                                         \
@@ -307,9 +316,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nPair = (p.nQT + 1) / 2;
   const F2Unit un(p);
-  const int pair = un.unit % nPair;
-  const int g = (un.unit / nPair) % p.G;
-  const int b = un.unit / (nPair * p.G);
+  const int b = un.unit % p.B;
+  const int pair = (un.unit / p.B) % nPair;
+  const int g = un.unit / (nPair * p.B);
   const int t0 = 2 * pair * p.npos;  // first position of the pair
   const int qpos_min = p.input_pos + t0;
   const int qpos_max = p.input_pos + min(t0 + 2 * p.npos, p.T) - 1;
@@ -394,7 +403,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const int32_t* pos_row = p.pos + bg * p.nT * F2_T;
       uint32_t seq = 0;
       bool ok = true;
-      F2_TRACE_DECL(lane == 0);
+      F2_TRACE_DECL(3, lane == 0);
       int4 pv_next = make_int4(0, 0, 0, 0);
       {
         int tf = un.t_lo;
@@ -450,7 +459,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       constexpr uint32_t idesc_qk = make_idesc_bf16(F2_T, F2_T, 0, 0);  // Q, K both K-major
       constexpr uint32_t idesc_pv = make_idesc_bf16(F2_T, HD, 0, 1);    // P K-major (TMEM), V MN-major
       bool ok = true;
-      F2_TRACE_DECL(true);
+      F2_TRACE_DECL(0, true);
       for (int w = 0; w < 2 && ok; ++w) ok = mbar_wait_bounded(&q_full[w], 0, abort_flag, p.status, STATUS_TIMEOUT_FULL);
       tc_fence_after();
       // stages are used in the order K0 V0 K1 V1 ...: tile i reads K from sequence number 2i and V from 2i + 1
@@ -570,7 +579,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     bool ok = n_active > 0;
     float m_used = -1e30f, l = 0.f;
     int i = 0;
-    F2_TRACE_DECL((warp == 2 || warp == 6) && lane == 0);  // the first warp of each warpgroup records
+    F2_TRACE_DECL(1 + wg, (warp == 2 || warp == 6) && lane == 0);  // the first warp of each warpgroup records
     {
       const int tf = next_active(un.t_lo - 1);
       if (ok && tf < un.t_hi && (tile_bits(tf) & 2u)) request_positions(tf);
@@ -833,11 +842,10 @@ __global__ void __launch_bounds__(256) flash_merge_kernel(const F2Params p) {
   const long long unit = p.n_full + r / (TILES * F2_T);
   if (unit >= (long long)p.B * p.G * nU) return;
   const int urow = (int)(r % (TILES * F2_T)), row = urow % F2_T;
-  const int qt = TILES * (int)(unit % nU) + urow / F2_T;
+  const int qt = TILES * (int)(unit / p.B % nU) + urow / F2_T;
   if (qt >= p.nQT) return;
-  const long long bg = unit / nU;
-  const long long wrow = (bg * p.nQT + qt) * F2_T + row;  // index into (B, G, nQT, 128)
-  const int g = (int)(bg % p.G), b = (int)(bg / p.G);
+  const int b = (int)(unit % p.B), g = (int)(unit / p.B / nU);
+  const long long wrow = (((long long)b * p.G + g) * p.nQT + qt) * F2_T + row;  // index into (B, G, nQT, 128)
   const int pl = row / p.gs, hq = row % p.gs;
   const int tq = qt * p.npos + pl;
   const bool row_valid = row < p.rows_used && tq < p.T;
@@ -924,9 +932,9 @@ flash256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const F2Unit un(p);
-  const int qt = un.unit % p.nQT;
-  const int g = (un.unit / p.nQT) % p.G;
-  const int b = un.unit / (p.nQT * p.G);
+  const int b = un.unit % p.B;
+  const int qt = (un.unit / p.B) % p.nQT;
+  const int g = un.unit / (p.nQT * p.B);
   const int t0 = qt * p.npos;
   const int qpos_min = p.input_pos + t0;
   const int qpos_max = p.input_pos + min(t0 + p.npos, p.T) - 1;
@@ -1555,34 +1563,37 @@ extern "C" int kvb_sdpa_fwd_set_trace(void* buf) {
   return KVB_OK;
 }
 
-// Scratch layout (int32 words, 16-byte aligned parts), provided by the caller:
-//   tile_min (B*G*nT) | tile_max (B*G*nT) | positions (B*G*nT*128) | lse2 (B*G*nQT*128 floats)
 // Units of a launch that are divided over the KV axis: those of a last wave that would leave half of the SMs or more idle,
 // when the cache is long enough. Whole waves stay undivided (no partial results to write and merge), the rest gets as many
 // CTAs as there are SMs, of at least 4 KV tiles each (a CTA's start, its partial results and their merge cost about two).
-// 2 x 499 queries x 40 heads over 7919 slots (160 units): the 12 of the second wave as 12 x 12 CTAs, flash 315 -> 189 us,
-// the call 446 -> 329.
+// Every sequence has the same units divided, so that equal sequences of a batch give equal bits (an evicting cache then drops
+// the same slots); up to B - 1 SMs of the whole waves stay without an undivided unit for that and take divided ones.
+// 2 x 499 queries x 40 heads over 7919 slots (160 units): the 12 of the second wave as 12 x 12 CTAs, the call
+// 399 -> 315 us. 256 queries x 32 heads over 4096 slots (32 units, four parts each): 95 -> 61 us.
 struct F2Split {
-  long long n_full;
+  long long units, n_full;  // of all sequences
   int n_split;
-  F2Split(long long units, long long nT) : n_full(units), n_split(1) {
+  F2Split(long long B, long long units_of_one, long long nT) : units(B * units_of_one), n_full(units), n_split(1) {
     static const int enabled = [] {
       const char* e = getenv("KVB200_F2_SPLIT");  // "0" switches the split off (diagnostics)
       return (e && e[0] == '0') ? 0 : 1;
     }();
-    const long long rest = units > 0 ? units % 148 : 0;
-    if (!enabled || rest == 0 || rest * 2 > 148 || nT < 16) return;
-    long long n = 148 / rest;
+    if (!enabled || units % 148 == 0 || nT < 16) return;
+    const long long whole = units / 148 * 148 / B * B, divided = units - whole;
+    if (divided * 2 > 148) return;
+    long long n = 148 / divided;
     if (n > nT / 4) n = nT / 4;
     if (n > 16) n = 16;
     if (n < 2) return;
-    n_full = units - rest;
+    n_full = whole;
     n_split = (int)n;
   }
-  long long part_rows(long long units, int rows) const { return (units - n_full) * n_split * rows; }
+  long long part_rows(int rows) const { return (units - n_full) * n_split * rows; }
 };
 
-//   ... | partial results of the divided units: part_lse2 (a float per row) | part_o (a row of floats each)
+// Scratch layout (int32 words, 16-byte aligned parts), provided by the caller:
+//   tile_min (B*G*nT) | tile_max (B*G*nT) | positions (B*G*nT*128) | lse2 (B*G*nQT*128 floats)
+//   | partial results of the divided units: part_lse2 (a float per row) | part_o (a row of floats each)
 extern "C" long long kvb_sdpa_fwd_scratch_bytes(int B, int H, int G, int q_len, int kv_len) {
   if (G <= 0 || H % G || H / G > 128) return -1;
   const int gs = H / G;
@@ -1592,8 +1603,7 @@ extern "C" long long kvb_sdpa_fwd_scratch_bytes(int B, int H, int G, int q_len, 
   const long long bgt = kvb::f2_round4((long long)B * G * nT);
   long long words = 2 * bgt + (long long)B * G * nT * 128 + (long long)B * G * nQT * 128;
   // pairs of query tiles (head size 64, 128) or single ones (256), whichever needs more
-  const long long pairs = (long long)B * G * ((nQT + 1) / 2), tiles = (long long)B * G * nQT;
-  const long long r2 = F2Split(pairs, nT).part_rows(pairs, 256), r3 = F2Split(tiles, nT).part_rows(tiles, 128);
+  const long long r2 = F2Split(B, G * ((nQT + 1) / 2), nT).part_rows(256), r3 = F2Split(B, G * nQT, nT).part_rows(128);
   const long long w2 = kvb::f2_round4(r2) + r2 * 128, w3 = kvb::f2_round4(r3) + r3 * 256;
   return (words + (w2 > w3 ? w2 : w3)) * 4;
 }
@@ -1668,12 +1678,12 @@ extern "C" int kvb_sdpa_fwd_ex(const void* q, const void* k, const void* v, cons
 
   f2_prepare_kernel<<<B * G * p.nT, F2_T, 0, s>>>(token_pos, tmin, tmax, pos, G, kv_len, p.nT, tp_sb, tp_sg);
   const int nPair = head_size == 256 ? p.nQT : (p.nQT + 1) / 2;  // head size 256: one query tile per CTA
-  const F2Split split((long long)B * G * nPair, p.nT);
+  const F2Split split(B, (long long)G * nPair, p.nT);
   p.n_full = (int)split.n_full;
   p.n_split = split.n_split;
   p.tiles_per_split = (p.nT + p.n_split - 1) / p.n_split;
   p.part_lse2 = lse2 + (long long)B * G * p.nQT * 128;
-  p.part_o = p.part_lse2 + f2_round4(split.part_rows((long long)B * G * nPair, head_size == 256 ? 128 : 256));
+  p.part_o = p.part_lse2 + f2_round4(split.part_rows(head_size == 256 ? 128 : 256));
   const bool gen = window > 0 || softcap > 0.f;
   if (head_size == 256) return f3_launch(tmQ, tmK, tmV, p, gen, s);
   if (head_size == 128) return gen ? f2_launch<true, 128>(tmQ, tmK, tmV, p, s) : f2_launch<false, 128>(tmQ, tmK, tmV, p, s);

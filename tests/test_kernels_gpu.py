@@ -320,6 +320,18 @@ def test_sdpa_divides_only_the_last_wave(B, H, G, T, L, mode, D):
     _sdpa_case(B, H, G, T, L, 3 * L if mode == "perm" else L - T, mode, D=D)
 
 
+@pytest.mark.parametrize("B,H,G,T,L,D", [
+    (2, 40, 8, 499, 2100, 128),    # 160 units: 74 of each sequence in one wave, 6 divided
+    (3, 40, 8, 331, 2100, 128),    # 168 units: 49 of each in 147 SMs, 7 divided
+    (5, 8, 8, 1100, 2100, 64),     # 200 units: 29 of each in 145 SMs, 11 divided
+    (2, 8, 4, 1211, 2500, 256)])   # 152 units of one query tile: 74 of each, 2 divided
+def test_sdpa_equal_sequences_of_a_batch_give_equal_bits(B, H, G, T, L, D):
+    q, k, v = (torch.randn(1, n, t, D, device=DEV, dtype=torch.bfloat16).expand(B, n, t, D).contiguous() for n, t in ((H, T), (G, L), (G, L)))
+    for res in _cuda().sdpa_fwd(q, k, v, D**-0.5, L - T, None, True):
+        assert all(torch.equal(res[b], res[0]) for b in range(1, B))
+    _cuda().check_status(DEV)
+
+
 @pytest.mark.parametrize("D", [128, 64])
 def test_sdpa_reads_a_slice_of_positions_in_place(D):
     """The queries of a chunk are a slice of the cell's (B,H,T',D) tensor: forward and backward read it through the
