@@ -790,7 +790,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                               __uint_as_float(o[4 * u + 2]) * inv_l, __uint_as_float(o[4 * u + 3]) * inv_l);
           }
         }
-        if (row_valid) p.part_lse2[prow] = l > 0.f ? lse2 : -INFINITY;
+        if (row_valid) p.part_lse2[prow] = l == 0.f ? -INFINITY : lse2;  // NaN scores: +inf
       } else {
       // tcgen05.ld is warp-collective: rows without a query take part in the loads and skip the stores
       __nv_bfloat16* dst = p.out + (((long long)b * p.T + (row_valid ? tq : 0)) * p.H + (g * p.gs + (row_valid ? hq : 0))) * HD;
@@ -857,7 +857,7 @@ __global__ void __launch_bounds__(256) flash_merge_kernel(const F2Params p) {
   const long long prow = (unit - p.n_full) * p.n_split * (TILES * F2_T) + urow;
   const float lse_s = lane < p.n_split ? p.part_lse2[prow + (long long)lane * (TILES * F2_T)] : -INFINITY;
   const float mx = warp_max(lse_s);
-  const float w_s = lse_s > -INFINITY ? exp2f(lse_s - mx) : 0.f;
+  const float w_s = lse_s > -INFINITY ? exp2f(lse_s - mx) : 0.f;  // NaN for a split with NaN scores
   const float total = warp_sum(w_s);
   constexpr int PER = HD / 32;
   float acc[PER];
@@ -869,9 +869,11 @@ __global__ void __launch_bounds__(256) flash_merge_kernel(const F2Params p) {
     const float2* src = reinterpret_cast<const float2*>(p.part_o + (prow + (long long)sidx * (TILES * F2_T)) * HD + PER * lane);
 #pragma unroll
     for (int e = 0; e < PER / 2; ++e) {
+      // A split of which the row sees nothing adds nothing, whatever it holds: an infinite value hidden from this row makes the
+      // zero weights of the split NaN.
       const float2 o = src[e];
-      acc[2 * e] += w * o.x;
-      acc[2 * e + 1] += w * o.y;
+      acc[2 * e] = w == 0.f ? acc[2 * e] : fmaf(w, o.x, acc[2 * e]);
+      acc[2 * e + 1] = w == 0.f ? acc[2 * e + 1] : fmaf(w, o.y, acc[2 * e + 1]);
     }
   }
   const float inv = total > 0.f ? 1.f / total : 0.f;
@@ -1213,7 +1215,7 @@ flash256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                               __uint_as_float(o[4 * u + 2]) * inv_l, __uint_as_float(o[4 * u + 3]) * inv_l);
           }
         }
-        if (row_valid) p.part_lse2[prow] = l > 0.f ? lse2 : -INFINITY;
+        if (row_valid) p.part_lse2[prow] = l == 0.f ? -INFINITY : lse2;  // NaN scores: +inf
       } else {
         __nv_bfloat16* dst = p.out + (((long long)b * p.T + tqv) * p.H + h) * F3_HD;
 #pragma unroll 1

@@ -332,6 +332,27 @@ def test_sdpa_equal_sequences_of_a_batch_give_equal_bits(B, H, G, T, L, D):
     _cuda().check_status(DEV)
 
 
+@pytest.mark.parametrize("D", [64, 128, 256])
+def test_sdpa_parts_keep_infinite_values_from_rows_that_do_not_see_them(D):
+    """One group of 64 KV tiles in 16 parts. The last part holds only tokens that the first 100 rows do not see; one of their
+    values is infinite (its zero weights times infinity are NaN there). A NaN key makes every row that sees it NaN."""
+    T, L, new = 128, 8192, 1 << 20
+    q, k, v = (torch.randn(1, 1, n, D, device=DEV, dtype=torch.bfloat16) for n in (T, L, L))
+    tp = torch.arange(L, device=DEV, dtype=torch.int32)
+    tp[:100] = torch.arange(new, new + 100, device=DEV)
+    tp[-512:] = torch.iinfo(torch.int32).max - 1
+    tp[-28:] = torch.arange(new + 100, new + T, device=DEV)
+    want, _, want_lse = _cuda().sdpa_fwd(q, k, v, D**-0.5, new, tp)
+    v[:, :, -1] = math.inf
+    out, _, lse = _cuda().sdpa_fwd(q, k, v, D**-0.5, new, tp)
+    assert torch.equal(out[:, :100], want[:, :100]) and torch.equal(lse, want_lse)
+    assert not out[:, -1].isfinite().any()
+    k[:, :, 50] = math.nan  # position new + 50
+    out = _cuda().sdpa_fwd(q, k, v, D**-0.5, new, tp)[0]
+    assert torch.equal(out[:, :50], want[:, :50]) and out[:, 50:].isnan().all()
+    _cuda().check_status(DEV)
+
+
 @pytest.mark.parametrize("D", [128, 64])
 def test_sdpa_reads_a_slice_of_positions_in_place(D):
     """The queries of a chunk are a slice of the cell's (B,H,T',D) tensor: forward and backward read it through the
