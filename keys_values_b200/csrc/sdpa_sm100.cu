@@ -1567,15 +1567,16 @@ extern "C" int kvb_sdpa_fwd_set_trace(void* buf) {
 
 // Units of a launch that are divided over the KV axis: those of a last wave that would leave half of the SMs or more idle,
 // when the cache is long enough. Whole waves stay undivided (no partial results to write and merge), the rest gets as many
-// CTAs as there are SMs, of at least 4 KV tiles each (a CTA's start, its partial results and their merge cost about two).
+// CTAs as there are SMs, of equally many KV tiles, at least 4 (a CTA's start, its partial results and their merge cost about
+// two); the last part of a unit takes what is left. Where the rounding up leaves parts without any tile, there are fewer parts.
 // Every sequence has the same units divided, so that equal sequences of a batch give equal bits (an evicting cache then drops
 // the same slots); up to B - 1 SMs of the whole waves stay without an undivided unit for that and take divided ones.
-// 2 x 499 queries x 40 heads over 7919 slots (160 units): the 12 of the second wave as 12 x 12 CTAs, the call
+// 2 x 499 queries x 40 heads over 7919 slots (160 units): the 12 of the second wave as 12 x 11 CTAs, the call
 // 399 -> 315 us. 256 queries x 32 heads over 4096 slots (32 units, four parts each): 95 -> 61 us.
 struct F2Split {
   long long units, n_full;  // of all sequences
-  int n_split;
-  F2Split(long long B, long long units_of_one, long long nT) : units(B * units_of_one), n_full(units), n_split(1) {
+  int n_split, tiles;           // parts of a divided unit, KV tiles of a part
+  F2Split(long long B, long long units_of_one, long long nT) : units(B * units_of_one), n_full(units), n_split(1), tiles((int)nT) {
     static const int enabled = [] {
       const char* e = getenv("KVB200_F2_SPLIT");  // "0" switches the split off (diagnostics)
       return (e && e[0] == '0') ? 0 : 1;
@@ -1588,7 +1589,8 @@ struct F2Split {
     if (n > 16) n = 16;
     if (n < 2) return;
     n_full = whole;
-    n_split = (int)n;
+    tiles = (int)((nT + n - 1) / n);
+    n_split = (int)((nT + tiles - 1) / tiles);
   }
   long long part_rows(int rows) const { return (units - n_full) * n_split * rows; }
 };
@@ -1683,7 +1685,7 @@ extern "C" int kvb_sdpa_fwd_ex(const void* q, const void* k, const void* v, cons
   const F2Split split(B, (long long)G * nPair, p.nT);
   p.n_full = (int)split.n_full;
   p.n_split = split.n_split;
-  p.tiles_per_split = (p.nT + p.n_split - 1) / p.n_split;
+  p.tiles_per_split = split.tiles;
   p.part_lse2 = lse2 + (long long)B * G * p.nQT * 128;
   p.part_o = p.part_lse2 + f2_round4(split.part_rows(head_size == 256 ? 128 : 256));
   const bool gen = window > 0 || softcap > 0.f;

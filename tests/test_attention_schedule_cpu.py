@@ -2,6 +2,8 @@
 import re
 from pathlib import Path
 
+import pytest
+
 CSRC = Path(__file__).resolve().parent.parent / "keys_values_b200" / "csrc"
 
 
@@ -81,3 +83,33 @@ def test_issuers_of_the_backward_never_miss_a_phase():
     stalls, wrong = _reachable_stalls(6, _turns())
     assert not stalls and not wrong
     assert _reachable_stalls(4, 1)[0]  # one barrier alone can be overrun: issuer A arrives twice before issuer B has looked
+
+
+def _division(B, units, nT):
+    """Units (of ``B * units``) that a forward launch divides over the KV axis and their parts: a last wave at most half full, as many
+    of every sequence, parts of equally many KV tiles, four at least, but for a shorter last one."""
+    whole = B * units // 148 * 148 // B * B
+    divided = B * units - whole
+    if B * units % 148 == 0 or nT < 16 or 2 * divided > 148:
+        return 0, 1
+    tiles = -(-nT // min(148 // divided, nT // 4, 16))
+    return divided, -(-nT // tiles)
+
+
+@pytest.mark.parametrize("B,H,G,T,L,want", [
+    (1, 32, 8, 256, 4096, (32, 4)),    # 32 KV tiles: parts of 8
+    (2, 40, 8, 499, 7919, (12, 11)),   # 74 units of each sequence in a wave; 62 KV tiles in parts of 6 (12 would leave one empty)
+    (1, 4, 1, 33, 2100, (1, 4)),       # 17 KV tiles: parts of 5, the last of 2
+    (1, 4, 1, 33, 8192, (1, 16)),      # 64 KV tiles: parts of 4
+    (3, 40, 8, 331, 2100, (21, 4)),    # 49 of each sequence in 147 SMs
+    (1, 32, 8, 1024, 16384, (0, 1)), (1, 4, 1, 33, 1900, (0, 1))])  # a wave more than half full; a short cache
+def test_partial_results_have_room_for_the_parts_that_are_launched(B, H, G, T, L, want):
+    """Scratch of a forward call: tile ranges, positions, normalisers, and the rows of every part (a normaliser and the features),
+    for pairs of query tiles or, at head size 256, for single ones."""
+    from keys_values_b200.ops import cuda
+
+    nT, nQT = -(-L // 128), -(-T // (128 // (H // G)))
+    assert _division(B, G * -(-nQT // 2), nT) == want
+    parts = [(n * p, rows, D) for (n, p), rows, D in ((want, 256, 128), (_division(B, G * nQT, nT), 128, 256))]
+    words = 2 * -(-B * G * nT // 4) * 4 + B * G * (nT + nQT) * 128 + max(n * rows * (1 + D) for n, rows, D in parts)
+    assert cuda.lib().kvb_sdpa_fwd_scratch_bytes(B, H, G, T, L) == 4 * words
