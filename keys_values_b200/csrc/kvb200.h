@@ -106,8 +106,16 @@ int kvb_sdpa_fwd_ex(const void* q, const void* k, const void* v, const int32_t* 
                     long long k_sb, long long k_sg, long long tp_sb, long long tp_sg, float scale, int input_pos, int window,
                     float softcap, int* status, void* stream);
 
-// ---- sdpa_bwd_sm100.cu: dq (B,H,T,D) bf16 is written, dk/dv (B,G,C,D) fp32 are accumulated into
+// ---- sdpa_bwd_sm100.cu: dq (B,H,T,D) bf16 is written, dk/dv (B,G,C,D) fp32 are accumulated into.
+// Most of the scratch holds dS, up to 1 GiB; the two calls that end in _within take another limit in bytes (0: 1 GiB; less than
+// 32 KB per 128 slots counts as that) and work in more rounds. launches: number of kernels launched, or NULL.
 long long kvb_sdpa_bwd_scratch_bytes(int B, int H, int G, int q_len, int kv_len);
+long long kvb_sdpa_bwd_scratch_bytes_within(int B, int H, int G, int q_len, int kv_len, long long ds_limit);
+int kvb_sdpa_bwd_within(const void* q, const void* k, const void* v, const int32_t* token_pos, const void* out, const void* dout,
+                        const float* lse, void* dq, float* dk, float* dv, void* scratch, int B, int H, int G, int q_len,
+                        int kv_len, int head_size, long long q_sb, long long q_sh, long long k_sb, long long k_sg,
+                        long long tp_sb, long long tp_sg, long long dk_sb, long long dk_sg, float scale, int input_pos,
+                        int window, float softcap, long long ds_limit, int* launches, int* status, void* stream);
 int kvb_sdpa_bwd(const void* q, const void* k, const void* v, const int32_t* token_pos, const void* out, const void* dout,
                  const float* lse, void* dq, float* dk, float* dv, void* scratch, int B, int H, int G, int q_len, int kv_len,
                  long long k_sb, long long k_sg, long long tp_sb, long long tp_sg, long long dk_sb, long long dk_sg, float scale,

@@ -20,7 +20,8 @@
 // dS passes through memory (32 KB written and read per tile) instead of being reduced into dQ by atomics: a coalesced
 // red.add.f32 of the 64 KB dQ tile was measured at 5.9 TB/s over the chip, no faster than the two 32 KB passes, and its
 // order is not fixed. Every output has one owner and a fixed order of sums: gradients are the same run to run.
-// The workspace is bounded (BO_DS_LIMIT): larger calls go in rounds over query tiles, then over (sequence, group) pairs.
+// The workspace is bounded (BO_DS_LIMIT, or what the caller has): larger calls go in rounds over query tiles, then over
+// (sequence, group) pairs.
 //
 // Replaces the blocked fp32 PyTorch backward of the reference
 // (keys_values/attention/sdpa_op.py:31-251) and the library SDPA backward it otherwise uses.
@@ -697,15 +698,15 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const BoParams p) {
   }
 }
 
-// Rounds of one call. A round's workspace is pairs · nT · nq tiles of 32 KB; it is kept below 1 GiB, the dS of a chunk of
-// 1024 queries x 32 heads over 16384 slots. Query tiles are divided first: every round then still has all (pair, KV tile)
-// CTAs, so its last wave stays as full as that of one launch. Below 8 query tiles a round would mostly load and store its
-// K, V, dK and dV tiles, and the pairs are divided as well.
+// Rounds of one call. A round's workspace is pairs · nT · nq tiles of 32 KB; it is kept below a limit, by default 1 GiB, the dS of
+// a chunk of 1024 queries x 32 heads over 16384 slots. Query tiles are divided first: every round then still has all (pair, KV
+// tile) CTAs, so its last wave stays as full as that of one launch. Below 8 query tiles a round would mostly load and store its
+// K, V, dK and dV tiles, and the pairs are divided as well. The least round is one query tile of one pair (32 KB per KV tile).
 constexpr long long BO_DS_LIMIT = 1LL << 30;
 struct BoRounds {
   int pairs, nq;
-  BoRounds(long long bg, long long nT, long long nQT) {
-    const long long tiles = BO_DS_LIMIT / BO_TILE;
+  BoRounds(long long bg, long long nT, long long nQT, long long limit) {
+    const long long tiles = (limit > 0 ? limit : BO_DS_LIMIT) / BO_TILE;
     const long long least = nQT < 8 ? nQT : 8;
     long long pr = tiles / (nT * least);
     pr = pr < 1 ? 1 : (pr > bg ? bg : pr);
@@ -723,8 +724,8 @@ struct BoLayout {  // scratch: tile_min | tile_max | statistics | head-major cop
   int npos, nT, nQT;
   BoRounds rounds;
   static long long round256(long long n) { return (n + 255) / 256 * 256; }
-  BoLayout(int B, int H, int G, int T, int L)
-      : npos(128 / (H / G)), nT((L + 127) / 128), nQT((T + npos - 1) / npos), rounds((long long)B * G, nT, nQT) {
+  BoLayout(int B, int H, int G, int T, int L, long long ds_limit)
+      : npos(128 / (H / G)), nT((L + 127) / 128), nQT((T + npos - 1) / npos), rounds((long long)B * G, nT, nQT, ds_limit) {
     stats = round256(2LL * B * G * nT * 4);
     dot = stats + (long long)B * G * nQT * 1024;
     ds = dot + round256((long long)B * H * T * 256);
@@ -756,15 +757,16 @@ static int bw_make_tmap_4d(CUtensorMap* tm, const void* ptr, uint64_t d0, uint64
   return r == CUDA_SUCCESS ? KVB_OK : KVB_ERR_TMAP;
 }
 
-// all launches of one call for one (GEN, head size) instantiation
+// all launches of one call for one (GEN, head size) instantiation; returns their number
 template <bool GEN, int HD>
-static void bo_launch(const CUtensorMap& tmQ, const CUtensorMap& tmO, const CUtensorMap& tmK, const CUtensorMap& tmV, BoParams p, int BG,
+static int bo_launch(const CUtensorMap& tmQ, const CUtensorMap& tmO, const CUtensorMap& tmK, const CUtensorMap& tmV, BoParams p, int BG,
                       const BoRounds& rounds, long long* trace, int trace_mode, cudaStream_t s) {
   static kvb::PerDeviceOnce attr_once;
   if (attr_once.first()) {
     cudaFuncSetAttribute(bwd_dkv_kernel<GEN, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, BoSmem::TOTAL);
     cudaFuncSetAttribute(bwd_dq_kernel<GEN, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, BoDqSmem::TOTAL);
   }
+  int launches = 0;
   for (int bg0 = 0; bg0 < BG; bg0 += rounds.pairs) {
     const int pairs = min(rounds.pairs, BG - bg0);
     for (int q0 = 0; q0 < p.nQT; q0 += rounds.nq) {
@@ -773,8 +775,10 @@ static void bo_launch(const CUtensorMap& tmQ, const CUtensorMap& tmO, const CUte
       bwd_dkv_kernel<GEN, HD><<<pairs * p.nT, BO_THREADS, BoSmem::TOTAL, s>>>(tmK, tmV, tmQ, tmO, p);
       p.trace = trace_mode == 0 ? trace : nullptr;
       bwd_dq_kernel<GEN, HD><<<pairs * p.nq, BO_DQ_THREADS, BoDqSmem::TOTAL, s>>>(tmK, p);
+      launches += 2;
     }
   }
+  return launches;
 }
 
 }  // namespace kvb
@@ -792,18 +796,25 @@ extern "C" int kvb_sdpa_bwd_set_trace(void* buf, int cap, int mode) {
   return KVB_OK;
 }
 
-extern "C" long long kvb_sdpa_bwd_scratch_bytes(int B, int H, int G, int q_len, int kv_len) {
+extern "C" long long kvb_sdpa_bwd_scratch_bytes_within(int B, int H, int G, int q_len, int kv_len, long long ds_limit) {
   if (B <= 0 || G <= 0 || q_len <= 0 || kv_len <= 0 || H < G || H / G > 64) return 16;  // refused by the call
-  return kvb::BoLayout(B, H, G, q_len, kv_len).total;
+  return kvb::BoLayout(B, H, G, q_len, kv_len, ds_limit).total;
+}
+extern "C" long long kvb_sdpa_bwd_scratch_bytes(int B, int H, int G, int q_len, int kv_len) {
+  return kvb_sdpa_bwd_scratch_bytes_within(B, H, G, q_len, kv_len, 0);
 }
 
 // head_size: 128 or 64; q_sb, q_sh: batch and head strides of q in elements (0, 0: contiguous (B,H,T,D)); window: sliding
-// window in tokens (0: none); softcap: logit soft-capping threshold (0: none), as in the forward.
+// window in tokens (0: none); softcap: logit soft-capping threshold (0: none), as in the forward. ds_limit: bytes of dS in
+// `scratch` (0: 1 GiB), the same as in the question for the scratch size; launches: their number, or NULL.
 extern "C" int kvb_sdpa_bwd_ex(const void* q, const void* k, const void* v, const int32_t* token_pos, const void* out,
                                const void* dout, const float* lse, void* dq, float* dk, float* dv, void* scratch, int B, int H,
                                int G, int q_len, int kv_len, int head_size, long long q_sb, long long q_sh, long long k_sb,
                                long long k_sg, long long tp_sb, long long tp_sg, long long dk_sb, long long dk_sg, float scale,
-                               int input_pos, int window, float softcap, int* status, void* stream);
+                               int input_pos, int window, float softcap, int* status, void* stream) {
+  return kvb_sdpa_bwd_within(q, k, v, token_pos, out, dout, lse, dq, dk, dv, scratch, B, H, G, q_len, kv_len, head_size, q_sb, q_sh,
+                             k_sb, k_sg, tp_sb, tp_sg, dk_sb, dk_sg, scale, input_pos, window, softcap, 0, nullptr, status, stream);
+}
 
 extern "C" int kvb_sdpa_bwd(const void* q, const void* k, const void* v, const int32_t* token_pos, const void* out,
                             const void* dout, const float* lse, void* dq, float* dk, float* dv, void* scratch, int B, int H,
@@ -813,11 +824,12 @@ extern "C" int kvb_sdpa_bwd(const void* q, const void* k, const void* v, const i
                          tp_sb, tp_sg, dk_sb, dk_sg, scale, input_pos, 0, 0.f, status, stream);
 }
 
-extern "C" int kvb_sdpa_bwd_ex(const void* q, const void* k, const void* v, const int32_t* token_pos, const void* out,
-                               const void* dout, const float* lse, void* dq, float* dk, float* dv, void* scratch, int B, int H,
-                               int G, int q_len, int kv_len, int head_size, long long q_sb, long long q_sh, long long k_sb,
-                               long long k_sg, long long tp_sb, long long tp_sg, long long dk_sb, long long dk_sg, float scale,
-                               int input_pos, int window, float softcap, int* status, void* stream) {
+extern "C" int kvb_sdpa_bwd_within(const void* q, const void* k, const void* v, const int32_t* token_pos, const void* out,
+                                   const void* dout, const float* lse, void* dq, float* dk, float* dv, void* scratch, int B, int H,
+                                   int G, int q_len, int kv_len, int head_size, long long q_sb, long long q_sh, long long k_sb,
+                                   long long k_sg, long long tp_sb, long long tp_sg, long long dk_sb, long long dk_sg, float scale,
+                                   int input_pos, int window, float softcap, long long ds_limit, int* launches, int* status,
+                                   void* stream) {
   using namespace kvb;
   if (B <= 0 || H <= 0 || G <= 0 || q_len <= 0 || kv_len <= 0 || H % G) return KVB_ERR_ARG;
   if (window < 0 || softcap < 0.f || (softcap > 0.f && scale <= 0.f)) return KVB_ERR_ARG;
@@ -833,7 +845,7 @@ extern "C" int kvb_sdpa_bwd_ex(const void* q, const void* k, const void* v, cons
     const char* e = getenv("KVB200_BWD_DOUT_T");  // "0": read dO in place (diagnostics)
     return (e && e[0] == '0') ? 0 : 1;
   }();
-  const BoLayout lay(B, H, G, q_len, kv_len);
+  const BoLayout lay(B, H, G, q_len, kv_len, ds_limit);
   uint8_t* sc = reinterpret_cast<uint8_t*>(scratch);
   BoParams p;
   p.G = G; p.H = H; p.T = q_len; p.L = kv_len; p.nT = lay.nT; p.nQT = lay.nQT;
@@ -873,6 +885,7 @@ extern "C" int kvb_sdpa_bwd_ex(const void* q, const void* k, const void* v, cons
   else bo_stats_kernel<64><<<blocks, 256, 0, s>>>(go, o, lse, stats, dOt, B, G, H, q_len, gs, p.npos, p.nQT, scale);
   const bool gen = window > 0 || softcap > 0.f;
   auto launch = head_size == 128 ? (gen ? bo_launch<true, 128> : bo_launch<false, 128>) : (gen ? bo_launch<true, 64> : bo_launch<false, 64>);
-  launch(tmQ, tmO, tmK, tmV, p, B * G, lay.rounds, g_bw_trace, g_bw_trace_mode, s);
+  const int n = launch(tmQ, tmO, tmK, tmV, p, B * G, lay.rounds, g_bw_trace, g_bw_trace_mode, s);
+  if (launches) *launches = 2 + n;
   return cudaGetLastError() == cudaSuccess ? KVB_OK : KVB_ERR_LAUNCH;
 }

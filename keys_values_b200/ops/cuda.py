@@ -48,6 +48,7 @@ def lib():
             )
         _LIB = ctypes.CDLL(str(LIB_PATH))
         _LIB.kvb_sdpa_fwd_scratch_bytes.restype = ctypes.c_longlong
+        _LIB.kvb_sdpa_bwd_scratch_bytes_within.restype = ctypes.c_longlong
     return _LIB
 
 
@@ -574,16 +575,30 @@ def _norm_token_pos(token_pos, B, G, L):
     return token_pos
 
 
+_DS_LIMITS = (0, 1 << 27, 1 << 24, 1)  # 0: the 1 GiB of the kernels; 1: one query tile of one (sequence, group) at a time
+
+
+def _sdpa_bwd_scratch(B, H, G, T, L, ds_limit, dev):
+    """``(scratch, ds_limit)`` of a backward call: where the device has no room, with a smaller dS and more rounds."""
+    for limit in (ds_limit,) if ds_limit else _DS_LIMITS:
+        nbytes = lib().kvb_sdpa_bwd_scratch_bytes_within(B, H, G, T, L, _ll(limit))
+        try:
+            return torch.empty(nbytes // 4, dtype=torch.int32, device=dev), limit
+        except torch.OutOfMemoryError:
+            if ds_limit or limit == _DS_LIMITS[-1]:
+                raise
+
+
 def sdpa_bwd(grad_out, query, key, value, out, lse, scale, input_pos, token_pos=None, dk_accum=None, dv_accum=None,
-             sliding_window=None, softcap=None):
+             sliding_window=None, softcap=None, ds_limit: int = 0):
     """Attention backward (tcgen05 kernels). Returns ``(dq, dk, dv)``: ``dq (B,H,T,D)`` in
     the dtype of ``query``; ``dk, dv`` fp32. If ``dk_accum/dv_accum`` (fp32, cache shaped,
     contiguous along the last two axes) are given, the gradients are *added* into their
-    first ``kv_len`` slots and ``None`` is returned for them."""
+    first ``kv_len`` slots and ``None`` is returned for them.
+    ``ds_limit``: bytes of the workspace for dS (0: up to 1 GiB, less where the device has no more to give)."""
     B, H, T, D = query.shape
     G, L = key.shape[1], key.shape[2]
     dev = query.device
-    lib().kvb_sdpa_bwd_scratch_bytes.restype = ctypes.c_longlong
     query = _rows_in_place(query)
     grad_out = grad_out.contiguous()
     out = out.contiguous()
@@ -597,17 +612,16 @@ def sdpa_bwd(grad_out, query, key, value, out, lse, scale, input_pos, token_pos=
     elif dk_accum.stride(3) != 1 or dk_accum.stride(2) != D or dk_accum.stride() != dv_accum.stride() or dk_accum.dtype != torch.float32:
         raise NativeError("sdpa_bwd: accumulators must be fp32 with contiguous rows and equal strides")
     dq = torch.empty((B, H, T, D), dtype=torch.bfloat16, device=dev)
-    nbytes = lib().kvb_sdpa_bwd_scratch_bytes(B, H, G, T, L)
-    scratch = torch.empty(nbytes // 4, dtype=torch.int32, device=dev)
+    scratch, ds_limit = _sdpa_bwd_scratch(B, H, G, T, L, ds_limit, dev)
+    launches = ctypes.c_int(0)
     st = status_word(dev)
-    _check(lib().kvb_sdpa_bwd_ex(_p(query), _p(key), _p(value), _p(token_pos), _p(out), _p(grad_out), _p(lse.contiguous()), _p(dq),
-                                 _p(dk_accum), _p(dv_accum), _p(scratch), B, H, G, T, L, int(D), _ll(query.stride(0)), _ll(query.stride(1)),
-                                 _ll(key.stride(0)), _ll(key.stride(1)),
-                                 _ll(token_pos.stride(0) if token_pos is not None else 0),
-                                 _ll(token_pos.stride(1) if token_pos is not None else 0),
-                                 _ll(dk_accum.stride(0)), _ll(dk_accum.stride(1)), ctypes.c_float(scale), int(input_pos),
-                                 int(sliding_window or 0), ctypes.c_float(softcap or 0.0), _p(st), _stream(query)), "sdpa_bwd")
-    _count(4)
+    _check(lib().kvb_sdpa_bwd_within(
+        _p(query), _p(key), _p(value), _p(token_pos), _p(out), _p(grad_out), _p(lse.contiguous()), _p(dq), _p(dk_accum), _p(dv_accum),
+        _p(scratch), B, H, G, T, L, int(D), _ll(query.stride(0)), _ll(query.stride(1)), _ll(key.stride(0)), _ll(key.stride(1)),
+        _ll(token_pos.stride(0) if token_pos is not None else 0), _ll(token_pos.stride(1) if token_pos is not None else 0),
+        _ll(dk_accum.stride(0)), _ll(dk_accum.stride(1)), ctypes.c_float(scale), int(input_pos), int(sliding_window or 0),
+        ctypes.c_float(softcap or 0.0), _ll(ds_limit), ctypes.byref(launches), _p(st), _stream(query)), "sdpa_bwd")
+    _count(launches.value)
     if own:
         return dq, dk_accum, dv_accum
     return dq, None, None

@@ -113,3 +113,22 @@ def test_partial_results_have_room_for_the_parts_that_are_launched(B, H, G, T, L
     parts = [(n * p, rows, D) for (n, p), rows, D in ((want, 256, 128), (_division(B, G * nQT, nT), 128, 256))]
     words = 2 * -(-B * G * nT // 4) * 4 + B * G * (nT + nQT) * 128 + max(n * rows * (1 + D) for n, rows, D in parts)
     assert cuda.lib().kvb_sdpa_fwd_scratch_bytes(B, H, G, T, L) == 4 * words
+
+
+@pytest.mark.parametrize("B,H,G,T,L", [(1, 32, 8, 2048, 16384), (5, 8, 8, 1000, 16384), (1, 40, 8, 421, 8192), (1, 1, 1, 1, 1), (1, 4, 1, 9, 1 << 23)])
+def test_workspace_of_the_backward_stays_below_its_limit(B, H, G, T, L):
+    """Beside dS the scratch of a backward call holds a copy of dO, statistics and tile ranges; dS takes one query tile of one (sequence,
+    group) at least."""
+    import ctypes
+
+    from keys_values_b200.ops import cuda
+
+    npos = 128 // (H // G)
+    nT, nQT = -(-L // 128), -(-T // npos)
+    other = -(-2 * B * G * nT * 4 // 256) * 256 + B * G * nQT * 1024 + -(-B * H * T * 256 // 256) * 256
+    whole = B * G * nT * nQT << 15
+    for limit in (0, 1 << 30, 1 << 27, 1 << 24, 1):
+        ds = cuda.lib().kvb_sdpa_bwd_scratch_bytes_within(B, H, G, T, L, ctypes.c_longlong(limit)) - other
+        assert ds % (nT << 15) == 0 and ds >= nT << 15
+        assert ds <= max(limit or 1 << 30, nT << 15)
+        assert ds == whole or whole > (limit or 1 << 30)

@@ -480,6 +480,44 @@ def test_sdpa_bwd_edges_and_rounds(B, H, G, T, L, mode, window, D):
             assert _rel_err(a[b:b + 1], r) < 1e-2 or (a[b].float() - r[0].float()).norm() < 1e-2 * math.sqrt(r.numel())
 
 
+@pytest.mark.parametrize("short_of_memory", [False, True])
+@pytest.mark.parametrize("B,H,G,T,L,window,softcap,D", [
+    (2, 8, 2, 700, 1000, None, None, 128), (1, 10, 2, 333, 900, 200, None, 128), (1, 8, 2, 300, 1500, 256, 3.0, 64)])
+def test_sdpa_bwd_with_a_small_workspace(B, H, G, T, L, window, softcap, D, short_of_memory, monkeypatch):
+    """Less room for dS than the call would take, by ``ds_limit`` or because the device refuses more: many rounds give the same dQ and,
+    but for the order of fp32 sums, the same dK and dV."""
+    q, k, v = (torch.randn(B, n, t, D, device=DEV, dtype=torch.bfloat16) for n, t in ((H, T), (G, L), (G, L)))
+    go = torch.randn(B, T, H * D, device=DEV, dtype=torch.bfloat16)
+    out, _, lse = _cuda().sdpa_fwd(q, k, v, D**-0.5, L - T, None, False, window, softcap)
+    args = (go, q, k, v, out, lse, D**-0.5, L - T, None, None, None, window, softcap)
+    want = _cuda().sdpa_bwd(*args)
+    nT, nQT = -(-L // 128), -(-T // (128 // (H // G)))
+    if short_of_memory:
+        empty = torch.empty
+
+        def refuse(*size, **kw):
+            if kw.get("dtype") == torch.int32 and 4 * size[0] > (1 << 23) + 600 * B * H * T:  # 8 MB of dS, dO and the statistics
+                raise torch.OutOfMemoryError("not enough memory (a test)")
+            return empty(*size, **kw)
+
+        monkeypatch.setattr(torch, "empty", refuse)
+        rounds = [_cuda().sdpa_bwd(*args)]
+    else:
+        rounds = []
+        for limit in (1, nT << 15, 3 * nT << 15, 8 * nT << 15):  # the least, one, three and eight query tiles of one (sequence, group)
+            before = _cuda().launch_count()
+            rounds.append(_cuda().sdpa_bwd(*args, ds_limit=limit))
+            at_once = max(limit // (nT << 15), 1)
+            per_pair = -(-nQT // at_once)
+            assert _cuda().launch_count() - before == 2 + 2 * B * G * per_pair
+    _cuda().check_status(DEV)
+    for got in rounds:
+        assert torch.equal(got[0], want[0])
+        for a, r in zip(got[1:], want[1:]):
+            # a few hundred additions into the running sums, each within 2^-23 of them; a lost round is of order 0.1 and more
+            assert _rel_err(a, r) < 1e-4
+
+
 @pytest.mark.parametrize("B,H,G,T,L,mode,window,softcap", [
     (1, 8, 2, 256, 2048, "perm", None, None), (2, 8, 2, 100, 1000, "perm", None, None), (1, 14, 2, 77, 900, "arange", None, None),
     (1, 32, 8, 700, 700, "arange", None, None), (1, 3, 1, 50, 200, "perm", None, None), (1, 8, 2, 300, 1500, "arange", 256, 3.0)])
