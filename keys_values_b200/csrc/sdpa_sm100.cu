@@ -84,28 +84,34 @@ struct F2Smem {
   static constexpr int QX = TF + F2_MAX_FLAG_TILES;             // [128 x 16] bf16, column 0 = 1: A operand of the bias step
   static constexpr int KX = QX + F2_BIAS_TILE_BYTES;            // per ring stage: [128 x 16] bf16, column 0 = 0 or -inf
   static constexpr int BAR = KX + F2_STAGES * F2_BIAS_TILE_BYTES;
-  static constexpr int TR = BAR + 256;  // diagnostics: 4 roles x (8 counters, clock of the last mark)
-  static constexpr int TOTAL = TR + 160;
+  static constexpr int TOTAL = BAR + 256;
 };
 static_assert(F2Smem::TOTAL <= 232448, "shared memory of the flash kernel exceeds the limit of a CTA");
 
+// Units are query-tile pairs of a group (single tiles at head size 256), numbered (sequence, group, tile). In the grid they come
+// with the sequence fastest, so that a run of them holds as many of every sequence.
+template <typename P>
+__device__ __forceinline__ int f2_unit(const P& p, int at) {
+  return p.B > 1 ? at % p.B * p.units + at / p.B : at;
+}
 // The unit of a CTA and the KV tiles that it takes: all of them, or the range of its split.
 struct F2Unit {
-  int unit, split, t_lo, t_hi;
+  int at, unit, split, t_lo, t_hi;
   bool part;
   template <typename P>
   __device__ __forceinline__ explicit F2Unit(const P& p) {
     const int k = (int)blockIdx.x - p.n_full;
     part = k >= 0;
-    unit = part ? p.n_full + k / p.n_split : (int)blockIdx.x;
+    at = part ? p.n_full + k / p.n_split : (int)blockIdx.x;
+    unit = f2_unit(p, at);
     split = part ? k % p.n_split : 0;
     t_lo = part ? split * p.tiles_per_split : 0;
     t_hi = part ? min(p.nT, t_lo + p.tiles_per_split) : p.nT;
   }
-  // row `row` of the unit (of `rows`) in the partial buffers
+  // row `row` of a split (of `rows`) in the partial buffers, which follow the grid
   template <typename P>
   __device__ __forceinline__ long long part_row(const P& p, int rows, int row) const {
-    return ((long long)(unit - p.n_full) * p.n_split + split) * rows + row;
+    return ((long long)(at - p.n_full) * p.n_split + split) * rows + row;
   }
 };
 
@@ -123,10 +129,9 @@ struct F2Params {
   int input_pos;
   int* status;
   long long* trace;          // optional phase profile of CTA 0: 4 roles x 8 cycle counters
-  // Units (query-tile pairs; single tiles at head size 256) in the order of the grid, numbered (group, tile, sequence): the first
-  // n_full, as many of every sequence, have one CTA each, the others n_split CTAs, each over tiles_per_split KV tiles. Those
-  // write normalised fp32 partial outputs and their log2 normalisers, which a merge kernel combines.
-  int n_full, n_split, tiles_per_split;
+  // The first n_full units of the grid, as many of every sequence, have one CTA each, the others n_split CTAs, each over
+  // tiles_per_split KV tiles. Those write normalised fp32 partial outputs and their log2 normalisers, which a merge kernel combines.
+  int units, n_full, n_split, tiles_per_split;  // units: of one sequence
   float* part_o;             // (units − n_full, n_split, rows of a unit, D)
   float* part_lse2;          // (units − n_full, n_split, rows of a unit), -inf for a split that saw no visible slot
   // Sliding window (0: none): a slot is visible to a query at position q iff q - window < token <= q.
@@ -149,28 +154,20 @@ __device__ __forceinline__ float f2_softcap(float s, float pre, float post) {
 }
 
 // Optional phase profile of CTA 0 (diagnostics): each role adds the cycles spent since its previous mark to one of
-// eight counters and writes them once at the end, so that the measurement costs a clock read per mark. The counters lie in
-// shared memory: the loops of the flash kernel have no registers for them (1024 queries x 32 heads over 16384 slots: 468 us with
-// the counters in registers, 464 so).
+// eight counters and writes them once at the end, so that the measurement costs a clock read per mark.
 // Roles: 0 MMA issuer, 1 / 2 first warp of softmax warpgroup 0 / 1, 3 producer.
 __device__ __forceinline__ uint32_t f2_clock() {
   uint32_t c;
   asm volatile("mov.u32 %0, %%clock;" : "=r"(c));
   return c;
 }
-#define F2_TRACE_DECL(role, active)                                                                    \
-  uint32_t* const tr_acc = reinterpret_cast<uint32_t*>(smem + F2Smem::TR) + 9 * (role);                \
-  const bool tr_on = p.trace != nullptr && blockIdx.x == 0 && (active);                                \
-  if (tr_on) {                                                                                         \
-    for (int k_ = 0; k_ < 8; ++k_) tr_acc[k_] = 0;                                                     \
-    tr_acc[8] = f2_clock();                                                                            \
-  }
+#define F2_TRACE_DECL(active) uint32_t tr_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}; const bool tr_on = p.trace != nullptr && blockIdx.x == 0 && (active); uint32_t tr_last = tr_on ? f2_clock() : 0u
 #define F2_MARK(k)                                \
   do {                                            \
     if (tr_on) {                                  \
       const uint32_t now_ = f2_clock();           \
-      tr_acc[k] += now_ - tr_acc[8];              \
-      tr_acc[8] = now_;                           \
+      tr_acc[k] += now_ - tr_last;                \
+      tr_last = now_;                             \
     }                                             \
   } while (0)
 #define F2_TRACE_STORE(role)                                                         \
@@ -316,9 +313,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nPair = (p.nQT + 1) / 2;
   const F2Unit un(p);
-  const int b = un.unit % p.B;
-  const int pair = (un.unit / p.B) % nPair;
-  const int g = un.unit / (nPair * p.B);
+  const int pair = un.unit % nPair;
+  const int g = (un.unit / nPair) % p.G;
+  const int b = un.unit / (nPair * p.G);
   const int t0 = 2 * pair * p.npos;  // first position of the pair
   const int qpos_min = p.input_pos + t0;
   const int qpos_max = p.input_pos + min(t0 + 2 * p.npos, p.T) - 1;
@@ -403,7 +400,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const int32_t* pos_row = p.pos + bg * p.nT * F2_T;
       uint32_t seq = 0;
       bool ok = true;
-      F2_TRACE_DECL(3, lane == 0);
+      F2_TRACE_DECL(lane == 0);
       int4 pv_next = make_int4(0, 0, 0, 0);
       {
         int tf = un.t_lo;
@@ -459,7 +456,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       constexpr uint32_t idesc_qk = make_idesc_bf16(F2_T, F2_T, 0, 0);  // Q, K both K-major
       constexpr uint32_t idesc_pv = make_idesc_bf16(F2_T, HD, 0, 1);    // P K-major (TMEM), V MN-major
       bool ok = true;
-      F2_TRACE_DECL(0, true);
+      F2_TRACE_DECL(true);
       for (int w = 0; w < 2 && ok; ++w) ok = mbar_wait_bounded(&q_full[w], 0, abort_flag, p.status, STATUS_TIMEOUT_FULL);
       tc_fence_after();
       // stages are used in the order K0 V0 K1 V1 ...: tile i reads K from sequence number 2i and V from 2i + 1
@@ -579,7 +576,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     bool ok = n_active > 0;
     float m_used = -1e30f, l = 0.f;
     int i = 0;
-    F2_TRACE_DECL(1 + wg, (warp == 2 || warp == 6) && lane == 0);  // the first warp of each warpgroup records
+    F2_TRACE_DECL((warp == 2 || warp == 6) && lane == 0);  // the first warp of each warpgroup records
     {
       const int tf = next_active(un.t_lo - 1);
       if (ok && tf < un.t_hi && (tile_bits(tf) & 2u)) request_positions(tf);
@@ -839,13 +836,14 @@ __global__ void __launch_bounds__(256) flash_merge_kernel(const F2Params p) {
   const int nU = (p.nQT + TILES - 1) / TILES;
   const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);  // row among those of the divided units
   const int lane = threadIdx.x & 31;
-  const long long unit = p.n_full + r / (TILES * F2_T);
-  if (unit >= (long long)p.B * p.G * nU) return;
+  const long long part = r / (TILES * F2_T);
+  if (p.n_full + part >= (long long)p.B * p.units) return;
+  const int unit = f2_unit(p, p.n_full + (int)part);
   const int urow = (int)(r % (TILES * F2_T)), row = urow % F2_T;
-  const int qt = TILES * (int)(unit / p.B % nU) + urow / F2_T;
+  const int qt = TILES * (unit % nU) + urow / F2_T;
   if (qt >= p.nQT) return;
-  const int b = (int)(unit % p.B), g = (int)(unit / p.B / nU);
-  const long long wrow = (((long long)b * p.G + g) * p.nQT + qt) * F2_T + row;  // index into (B, G, nQT, 128)
+  const int bg = unit / nU, g = bg % p.G, b = bg / p.G;
+  const long long wrow = ((long long)bg * p.nQT + qt) * F2_T + row;  // index into (B, G, nQT, 128)
   const int pl = row / p.gs, hq = row % p.gs;
   const int tq = qt * p.npos + pl;
   const bool row_valid = row < p.rows_used && tq < p.T;
@@ -854,7 +852,7 @@ __global__ void __launch_bounds__(256) flash_merge_kernel(const F2Params p) {
     return;
   }
   const int h = g * p.gs + hq;
-  const long long prow = (unit - p.n_full) * p.n_split * (TILES * F2_T) + urow;
+  const long long prow = part * p.n_split * (TILES * F2_T) + urow;
   const float lse_s = lane < p.n_split ? p.part_lse2[prow + (long long)lane * (TILES * F2_T)] : -INFINITY;
   const float mx = warp_max(lse_s);
   const float w_s = lse_s > -INFINITY ? exp2f(lse_s - mx) : 0.f;  // NaN for a split with NaN scores
@@ -943,9 +941,9 @@ flash256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const F2Unit un(p);
-  const int b = un.unit % p.B;
-  const int qt = (un.unit / p.B) % p.nQT;
-  const int g = un.unit / (p.nQT * p.B);
+  const int qt = un.unit % p.nQT;
+  const int g = (un.unit / p.nQT) % p.G;
+  const int b = un.unit / (p.nQT * p.G);
   const int t0 = qt * p.npos;
   const int qpos_min = p.input_pos + t0;
   const int qpos_max = p.input_pos + min(t0 + p.npos, p.T) - 1;
@@ -1526,7 +1524,7 @@ static int f2_launch(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUten
     cudaFuncSetAttribute(flash_fwd_kernel<GEN, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, F2Smem::TOTAL);
     cudaFuncSetAttribute(colsum_kernel<GEN, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, CsSmemT<HD>::TOTAL);
   }
-  const int divided = p.B * p.G * ((p.nQT + 1) / 2) - p.n_full;
+  const int divided = p.B * p.units - p.n_full;
   flash_fwd_kernel<GEN, HD><<<p.n_full + divided * p.n_split, F2_THREADS, F2Smem::TOTAL, s>>>(tmQ, tmK, tmV, p);
   if (divided > 0) flash_merge_kernel<HD><<<divided * (2 * F2_T / 8), 256, 0, s>>>(p);
   if (p.weights) colsum_kernel<GEN, HD><<<p.B * p.G * p.nT, CS_THREADS, CsSmemT<HD>::TOTAL, s>>>(tmQ, tmK, p);
@@ -1542,7 +1540,7 @@ static int f3_launch(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUten
     cudaFuncSetAttribute(colsum_kernel<false, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, CsSmemT<256>::TOTAL);
     cudaFuncSetAttribute(colsum_kernel<true, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, CsSmemT<256>::TOTAL);
   }
-  const int divided = p.B * p.G * p.nQT - p.n_full;
+  const int divided = p.B * p.units - p.n_full;
   flash256_fwd_kernel<<<p.n_full + divided * p.n_split, F3_THREADS, F3Smem::TOTAL, s>>>(tmQ, tmK, tmV, p);
   if (divided > 0) flash_merge_kernel<256><<<divided * (F2_T / 8), 256, 0, s>>>(p);
   if (p.weights) {
@@ -1691,7 +1689,8 @@ extern "C" int kvb_sdpa_fwd_ex(const void* q, const void* k, const void* v, cons
 
   f2_prepare_kernel<<<B * G * p.nT, F2_T, 0, s>>>(token_pos, tmin, tmax, pos, G, kv_len, p.nT, tp_sb, tp_sg);
   const int nPair = head_size == 256 ? p.nQT : (p.nQT + 1) / 2;  // head size 256: one query tile per CTA
-  const F2Split split(B, (long long)G * nPair, p.nT);
+  p.units = G * nPair;
+  const F2Split split(B, p.units, p.nT);
   p.n_full = (int)split.n_full;
   p.n_split = split.n_split;
   p.tiles_per_split = split.tiles;
