@@ -14,9 +14,10 @@
 //     thread A:  wait P(i)  -> dV += P(i) dO(i),  S(i+1)          thread B:  wait dS(i) -> dK += dS(i) Q(i),  dP(i+1)
 // so that the exponentials of a tile run under dK / dP and the products P (dP − δ) under dV / S. S goes in two halves of
 // 64 columns, so that the exponentials of one half overlap dV and the next S of the other. Measured: 0.81 ms back to back
-// under the power cap, 0.69 ms in short runs (dkv 0.48, dq 0.19). dkv: 3220 cycles a tile (2304 of MMA, of which shared
-// memory serves most; compute chain: exponentials 1300 of 1024 at the special-function rate, dS 550, its stores 700);
-// dq: 5.8 TB/s of dS.
+// under the power cap, 0.69 ms in short runs (dkv 0.48, dq 0.18). dkv: 3220 cycles a tile, 2304 of them MMA, of which shared
+// memory serves most. Marks of the first compute warp (kvb_sdpa_bwd_set_trace): stores of dS, wait and exponentials of the
+// first half 1380, exponentials of the second half 770 (512 at the special-function rate), wait for dP and dS 960.
+// dq: 1.1 GB of dS at 6.1 TB/s.
 // dS passes through memory (32 KB written and read per tile) instead of being reduced into dQ by atomics: a coalesced
 // red.add.f32 of the 64 KB dQ tile was measured at 5.9 TB/s over the chip, no faster than the two 32 KB passes, and its
 // order is not fixed. Every output has one owner and a fixed order of sums: gradients are the same run to run.
@@ -838,7 +839,7 @@ extern "C" int kvb_sdpa_bwd_within(const void* q, const void* k, const void* v, 
   if (q_sb == 0) q_sb = (long long)H * q_sh;
   if ((q_sb % 8) || (q_sh % 8) || q_sh < (long long)q_len * head_size) return KVB_ERR_ALIGN;
   const int gs = H / G;
-  if (gs > 64) return KVB_ERR_UNSUPPORTED;  // a 64-column unit of the dK/dV launch holds all heads of a group
+  if (gs > 64) return KVB_ERR_UNSUPPORTED;  // not tested beyond: such groups fill a tile with one position
   if ((k_sb % 8) || (k_sg % 8) || (dk_sb % 4) || (dk_sg % 4)) return KVB_ERR_ALIGN;
   cudaStream_t s = (cudaStream_t)stream;
   static const int dout_headmajor = [] {

@@ -30,15 +30,16 @@
 //     of plain causal attention) is compared element by element. Tiles that no query can see are skipped.
 //
 // Kernel B (colsum_kernel), per (batch, KV group, KV tile of 128 slots): S^T = K Q^T per query tile
-//   on tcgen05 (M = 128 slots, N = 128 query rows), four S^T buffers in TMEM. A thread owns one slot
-//   and adds exp2(S·c − lse_row) over the 128 query rows of every tile from registers: no shared
-//   memory, no atomics, no partial buffers, a fixed order (run-to-run identical eviction decisions).
+//   on tcgen05 (M = 128 slots, N = 128 query rows), four S^T buffers in TMEM, one per warpgroup. A thread
+//   owns one slot and adds exp2(S·c − lse_row) over the 128 query rows of every fourth tile from registers;
+//   the normalisers come by bulk copies, the four sums of a slot meet in shared memory at the end. No
+//   atomics, no partial buffers, a fixed order (run-to-run identical eviction decisions).
 //   Position-major query rows turn the causal mask of a slot into one threshold on the column index.
 //
 // Variants: head size 64 and 128 are template parameters of these kernels (HD), sliding window and logit soft-capping a
 // separate instantiation (GEN); head size 256 has its own flash kernel further down (flash256_fwd_kernel) and shares the
-// column-sum and merge kernels. Launches with few query tiles are split over the KV axis (fp32 partials, merged in a
-// fixed order by flash_merge_kernel).
+// column-sum and merge kernels. A last wave that would leave half of the SMs idle is divided over the KV axis (F2Split: fp32
+// partials, merged in a fixed order by flash_merge_kernel).
 //
 // Replaces FlashInfer prefill + Triton score-sum + K/V reordering + query padding of the reference
 // (keys_values/attention/flashinfer_wrapper.py:51-273, :367-510, csrc/kernels/sdpa_prefill.cu,
@@ -1579,7 +1580,7 @@ extern "C" int kvb_sdpa_fwd_set_trace(void* buf) {
 // Every sequence has the same units divided, so that equal sequences of a batch give equal bits (an evicting cache then drops
 // the same slots); up to B - 1 SMs of the whole waves stay without an undivided unit for that and take divided ones.
 // 2 x 499 queries x 40 heads over 7919 slots (160 units): the 12 of the second wave as 12 x 11 CTAs, the call
-// 399 -> 315 us. 256 queries x 32 heads over 4096 slots (32 units, four parts each): 95 -> 61 us.
+// 390 -> 308 us. 256 queries x 32 heads over 4096 slots (32 units, four parts each): 94 -> 61 us.
 struct F2Split {
   long long units, n_full;  // of all sequences
   int n_split, tiles;           // parts of a divided unit, KV tiles of a part

@@ -514,8 +514,8 @@ def sdpa_supported(query: torch.Tensor, key: torch.Tensor, sliding_window, softc
 
 
 def sdpa_bwd_supported(query: torch.Tensor, key: torch.Tensor, sliding_window, softcap) -> bool:
-    """Same shapes as the forward, with at most 64 query heads per KV head (a 64-column unit of the dK/dV launch
-    holds all heads of a group). Any group size: 5 (Qwen3-14B) packs 25 positions x 5 heads into the 128-row tile."""
+    """Same shapes as the forward but for head size 256, and at most 64 query heads per KV head (the kernels are not tested
+    with larger groups). Any group size up to that: 5 (Qwen3-14B) packs 25 positions x 5 heads into the 128-row tile."""
     return (sdpa_supported(query, key, sliding_window, softcap) and query.shape[-1] in (64, 128)
             and query.shape[1] // key.shape[1] <= 64)
 

@@ -74,7 +74,7 @@ def bench_sdpa(out, peaks):
 
 
 def bench_sdpa_bwd(out, peaks):
-    """Backward (dQ launch + dK/dV launch + delta kernel) on the training-chunk shapes: a chunk of
+    """Backward (tile ranges, statistics, dK/dV kernel, dQ kernel) on the training-chunk shapes: a chunk of
     ``q`` new tokens against a cache of ``kv`` slots in random slot order."""
     from keys_values_b200.ops import cuda as cu
 
